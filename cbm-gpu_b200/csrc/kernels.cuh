@@ -59,10 +59,13 @@ struct QueueState {
 struct FwdArgs {
   // rows in level order
   int32_t n_items;
+  const int4* meta;          // register kernel: one record per item (kernels below)
   const int32_t* node;       // node id per item; bit 31 set: node has children
   const int64_t* ptr;        // [n_items + 1]
   const uint32_t* ent;       // column | sign << 31
   const float* val;          // values (SCALE_VALUES) or null
+  const float* sval;         // s * m[col] per entry of ent (SCALE_DCOL*), or null: formed from mult
+  const float* csval;        // the same per entry of cent
   const int32_t* par;        // parent node id, -1 for children of the virtual root
   const int32_t* par_item;   // queue position of the parent's item, -1
   const int32_t* self_slot;  // internal-node slot of the item's node, -1 if leaf
@@ -78,8 +81,13 @@ struct FwdArgs {
   // state
   const float* mult;
   unsigned int* node_flag;   // [n_rows], ready epoch of internal nodes
-  unsigned int* chunk_flag;  // [n_chunks]
+  unsigned int* chunk_flag;  // [n_chunks], then one per presummed row
   QueueState* qs;
+  // register kernel: presummed rows (item, node, first entry, entries), longest
+  // first, and its kClaimQueues row counters, kClaimStride apart
+  int32_t n_pre;
+  const int4* pre;
+  unsigned int* claims;
   // operands
   const void* x;
   int64_t ldx;
@@ -88,12 +96,13 @@ struct FwdArgs {
   int32_t nvec;        // vectors per row (columns / V)
   int32_t ldp;         // floats per row of partial / parent-state scratch
   float* partial;      // [n_chunks, ldp]
+  float* pre_rows;     // [n_pre, ldp] sums of presummed rows, or null: kept in Y (FP32)
   float* pstate;       // [n_internal, ldp] fp32 parent rows when Y is bf16
   int32_t scale_mode;
   int32_t prop_mode;
   int32_t team;        // lanes per row: 1, 2, 4, 8, 16 or 32
-  int32_t rows_per_claim;       // level-0 rows a team takes per claim
-  int32_t rows_per_claim_deep;  // rows below level 0 a team takes per claim
+  int32_t rows_per_claim;       // staged kernel: level-0 rows a team takes per claim
+  int32_t rows_per_claim_deep;  // staged kernel: rows below level 0 a team takes per claim
   int32_t n_root;               // items [0, n_root) are level 0 (no parent)
   // staged kernel with several teams per warp: claims of one unit per team,
   // unit u = items [unit[u], unit[u + 1]) (at most 8), level-0 units balanced
@@ -283,124 +292,200 @@ __host__ __device__ constexpr int unroll_for() {
   return (32 / (VPL * V)) < 1 ? 1 : ((32 / (VPL * V)) > 8 ? 8 : (32 / (VPL * V)));
 }
 
-// acc += sum over entries [beg, end) of scale_k * X[col_k], UF entries' gathers
-// in flight per lane (0: unroll_for's choice); OFF32: X holds fewer than 2^32
-// elements, so a row's offset is 32-bit element arithmetic
-template <typename XT, int VPL, int V, int UF = 0, bool OFF32 = false>
-__device__ __forceinline__ void gather_range(float (&acc)[VPL][V], const XT* __restrict__ x, int64_t ldx, int nvec,
-                                             const uint32_t* __restrict__ ent, const float* __restrict__ val,
-                                             int64_t beg, int64_t end, int scale_mode,
-                                             const float* __restrict__ mult, float dv, int tl, int TL,
-                                             unsigned tmask) {
-  constexpr int U = UF > 0 ? UF : unroll_for<VPL, V>();
-  for (int64_t base = beg; base < end; base += TL) {
-    const int64_t idx = base + tl;
-    uint32_t e = 0;
-    float sc = 0.f;
-    if (idx < end) {
-      e = __ldg(ent + idx);
-      const uint32_t c = e & kColMask;
-      const float sgn = (e >> 31) ? -1.f : 1.f;
-      if (scale_mode == SCALE_SIGN) {
-        sc = sgn;
-      } else if (scale_mode == SCALE_DCOL) {
-        sc = sgn * __ldg(mult + c);
-      } else if (scale_mode == SCALE_DCOL_DROW) {
-        sc = __fmul_rn(sgn * __ldg(mult + c), dv);
-      } else {
-        sc = __ldg(val + idx);
+// ---- register kernel: gathers ---------------------------------------------------
+// V elements of T as loaded (16 bytes or one element), widened when consumed, so
+// a gather in flight costs no more registers than its bytes.
+template <typename T, int V>
+struct Raw;
+template <>
+struct Raw<float, 4> {
+  using type = float4;
+  static constexpr int regs = 4;
+  static __device__ __forceinline__ type zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
+  static __device__ __forceinline__ type load(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
+  static __device__ __forceinline__ void widen(const type& r, float (&o)[4]) {
+    o[0] = r.x; o[1] = r.y; o[2] = r.z; o[3] = r.w;
+  }
+};
+template <>
+struct Raw<float, 1> {
+  using type = float;
+  static constexpr int regs = 1;
+  static __device__ __forceinline__ type zero() { return 0.f; }
+  static __device__ __forceinline__ type load(const float* p) { return __ldg(p); }
+  static __device__ __forceinline__ void widen(const type& r, float (&o)[1]) { o[0] = r; }
+};
+template <>
+struct Raw<__nv_bfloat16, 8> {
+  using type = uint4;
+  static constexpr int regs = 4;
+  static __device__ __forceinline__ type zero() { return make_uint4(0u, 0u, 0u, 0u); }
+  static __device__ __forceinline__ type load(const __nv_bfloat16* p) {
+    return __ldg(reinterpret_cast<const uint4*>(p));
+  }
+  static __device__ __forceinline__ void widen(const type& r, float (&o)[8]) {
+    const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      o[2 * i] = __uint_as_float(w[i] << 16);
+      o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  }
+};
+template <>
+struct Raw<__nv_bfloat16, 1> {
+  using type = unsigned short;
+  static constexpr int regs = 1;
+  static __device__ __forceinline__ type zero() { return 0; }
+  static __device__ __forceinline__ type load(const __nv_bfloat16* p) {
+    return __ldg(reinterpret_cast<const unsigned short*>(p));
+  }
+  static __device__ __forceinline__ void widen(const type& r, float (&o)[1]) {
+    o[0] = __uint_as_float(((uint32_t)r) << 16);
+  }
+};
+
+// Gathers in flight per lane: 16 registers' worth (32 from four pieces per lane
+// on), at most 8.  Twice as many cost a resident block and were slower (GCN
+// graph, 128 BF16 columns: 152 -> 174 us, 64-column GIN 81 -> 90).
+template <typename XT, int VPL, int V>
+__host__ __device__ constexpr int reg_in_flight() {
+  const int u = (VPL >= 4 ? 32 : 16) / (VPL * Raw<XT, V>::regs);
+  return u < 1 ? 1 : (u > 8 ? 8 : u);
+}
+
+// Entry idx's scale before the row factor: s, the stored value, or s * m[col]
+// (from the plan's array when it has one).
+__device__ __forceinline__ float reg_scale(uint32_t e, const float* __restrict__ vals, int idx, int scale_mode,
+                                           const float* __restrict__ mult) {
+  const float sgn = (e >> 31) ? -1.f : 1.f;
+  if (scale_mode == SCALE_SIGN) return sgn;
+  if (vals) return __ldg(vals + idx);
+  return sgn * __ldg(mult + (e & kColMask));
+}
+
+// A lane's place in the rows of X: its first piece's address and, for each of
+// its VPL pieces, the byte offset from there (0 for a piece past the row's end:
+// the lane then reads its first piece again into sums no store reads; a lane
+// with no piece at all reads the row's first).  ldb: bytes between rows; WIDE
+// allows 2^32 of them and more.
+template <typename XT, int VPL, int V, bool WIDE>
+struct Lane {
+  const char* x;
+  uint32_t off[VPL];
+  uint32_t ldb, ldb_hi;
+  __device__ __forceinline__ Lane(const void* xv, int64_t ldx, int nvec, int tl, int TL) {
+    constexpr int piece = V * (int)sizeof(XT);
+    x = static_cast<const char*>(xv) + (tl < nvec ? tl * piece : 0);
+#pragma unroll
+    for (int v = 0; v < VPL; ++v) off[v] = tl + v * TL < nvec ? (uint32_t)(v * TL * piece) : 0u;
+    const uint64_t ld = (uint64_t)ldx * sizeof(XT);
+    ldb = (uint32_t)ld;
+    ldb_hi = (uint32_t)(ld >> 32);
+  }
+  __device__ __forceinline__ const char* row(uint32_t c) const {
+    const char* r = x + (uint64_t)c * ldb;
+    return WIDE ? r + ((uint64_t)(c * ldb_hi) << 32) : r;
+  }
+};
+
+// acc += sum of scale_k * X[col_k] over the `len` entries of ent, in order, one
+// FMA each.  Every lane of the warp calls it: the trip counts come from wlen,
+// the largest len of the warp's teams, so teams that share a warp step through
+// one instruction stream (a shuffle with per-team masks would split it), and a
+// team past its end is predicated off.  e / s: the lane's entry of the first
+// TL (loaded ahead by the caller); later batches of TL are loaded one batch
+// ahead.  `between` runs once, after the first group's gathers are issued and
+// before anything waits for them: the place for loads the next row needs, and
+// for an acquire, whose latency then hides under the gathers'.
+template <typename XT, int VPL, int V, int TLC, bool WIDE, typename Between>
+__device__ __forceinline__ void gather_row(float (&acc)[VPL][V], const Lane<XT, VPL, V, WIDE>& ln,
+                                           const uint32_t* __restrict__ ent, const float* __restrict__ vals, int len,
+                                           int wlen, uint32_t e, float s, float dv, int scale_mode,
+                                           const float* __restrict__ mult, int tl, int team_lanes, Between between) {
+  constexpr int U = reg_in_flight<XT, VPL, V>();
+  using R = Raw<XT, V>;
+  const int TL = TLC ? TLC : team_lanes;
+  if (wlen <= 0) {
+    between();
+    return;
+  }
+  for (int b = 0; b < wlen; b += TL) {
+    const int in = b + TL + tl;
+    uint32_t en = 0;
+    float sn = 0.f;
+    if (in < len) {
+      en = __ldg(ent + in);
+      if (vals) sn = __ldg(vals + in);
+    }
+    const uint32_t c = e & kColMask;
+    const int cnt = len - b < TL ? len - b : TL;   // this team's entries in the batch (<= 0: none)
+    const int wc = wlen - b < TL ? wlen - b : TL;  // the warp's
+    typename R::type raw[U][VPL];
+    auto load = [&](int j, int u) {
+      const char* row = ln.row(__shfl_sync(0xffffffffu, c, j + u, TL));
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) raw[u][v] = R::load(reinterpret_cast<const XT*>(row + ln.off[v]));
+    };
+    auto add = [&](float su, int u) {
+#pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        float t[V];
+        R::widen(raw[u][v], t);
+#pragma unroll
+        for (int k = 0; k < V; ++k) acc[v][k] = fmaf(su, t[k], acc[v][k]);
+      }
+    };
+    auto after_loads = [&](int j) {
+      if (b + j == 0) {
+        between();
+        s = __fmul_rn(s, dv);
+      }
+    };
+    int j = 0;
+    if (TLC == 32) {
+      // whole groups without predicates
+#pragma unroll 1
+      for (; j + U <= cnt; j += U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) load(j, u);
+        after_loads(j);
+#pragma unroll
+        for (int u = 0; u < U; ++u) add(__shfl_sync(0xffffffffu, s, j + u, TL), u);
       }
     }
-    const int cnt = (int)((end - base) < TL ? (end - base) : TL);
-    for (int j = 0; j < cnt; j += U) {
-      float buf[U][VPL][V];
-      float s[U];
+#pragma unroll 1
+    for (; j < wc; j += U) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const uint32_t eu = __shfl_sync(tmask, e, j + u < cnt ? j + u : 0, TL);
-        s[u] = __shfl_sync(tmask, sc, j + u < cnt ? j + u : 0, TL);
-        const XT* row = OFF32 ? x + (uint32_t)((eu & kColMask) * (uint32_t)ldx) : x + row_off(eu & kColMask, ldx);
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const int vi = tl + v * TL;
-          if (j + u < cnt && vi < nvec) {
-            Vec<XT, V>::load(row + (int64_t)vi * V, buf[u][v]);
-          } else {
-#pragma unroll
-            for (int k = 0; k < V; ++k) buf[u][v][k] = 0.f;
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
+        const char* row = ln.row(__shfl_sync(0xffffffffu, c, j + u, TL));
         if (j + u < cnt) {
 #pragma unroll
-          for (int v = 0; v < VPL; ++v)
-#pragma unroll
-            for (int k = 0; k < V; ++k) acc[v][k] = fmaf(s[u], buf[u][v][k], acc[v][k]);
+          for (int v = 0; v < VPL; ++v) raw[u][v] = R::load(reinterpret_cast<const XT*>(row + ln.off[v]));
         }
       }
+      after_loads(j);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float su = __shfl_sync(0xffffffffu, s, j + u, TL);
+        if (j + u < cnt) add(su, u);
+      }
     }
+    e = en;
+    if (!vals) sn = in < len ? reg_scale(en, vals, in, scale_mode, mult) : 0.f;
+    s = __fmul_rn(sn, dv);
   }
 }
 
-// Resident blocks per SM of the register kernel.  Rows of one 16-byte vector
-// per lane are latency-bound where X is L2-resident, and more warps hide more
-// of the latency, at the cost of registers (gathers in flight).  Measured on
-// B200, bit-identical results either way:
-//   X and Y of one type: 4 blocks (at most 64 registers) with two gathers in
-//     flight per lane (170K-node GCN graph: 128 BF16 columns 0.235 -> 0.210
-//     ms, 128 FP32 0.311 -> 0.258, 40 FP32 0.180 -> 0.162);
-//   BF16 X, FP32 Y: 3 blocks (at most 85 registers) where most rows wait on a
-//     parent (GCN graph, 40 columns: 0.160 ms against 0.196 with 2 blocks and
-//     0.210 with 4); WIDE, taken on shallower trees: 4 blocks with two in
-//     flight (512-graph batch, 64 columns: 4.87 ms against 5.44 with 3 blocks
-//     and 7.53 with 2).
-template <typename XT, typename YT, int VPL, bool COMP, bool WIDE>
+// Resident blocks per SM of the register kernel (registers per thread are
+// capped to fit them): four for full-warp rows of one vector per lane
+// (200,000-node power-law graph, 128 FP32 columns: 348 us with three, 295
+// with four), three where teams share a warp (40 BF16 columns on the GCN
+// graph: 103 against 121) and for two vectors per lane (47 scalar columns: 103
+// against 137 with two).
+template <typename XT, typename YT, int VPL, int FORM, int TLC>
 __host__ __device__ constexpr int fwd_min_blocks() {
-  return (VPL != 1 || COMP) ? 1 : ((sizeof(XT) == sizeof(YT) || WIDE) ? 4 : 3);
-}
-template <typename XT, typename YT, int VPL, bool COMP, bool WIDE>
-__host__ __device__ constexpr int fwd_in_flight() {
-  return fwd_min_blocks<XT, YT, VPL, COMP, WIDE>() == 4 ? 2 : 0;  // 0: unroll_for's choice
-}
-
-template <typename XT, typename YT, int VPL, int V, bool COMP = false, bool WIDE = false, bool OFF32 = false>
-__device__ __forceinline__ void fwd_chunk(const FwdArgs& a, int k, unsigned epoch, int tl, int TL, unsigned tmask) {
-  float acc[VPL][V];
-#pragma unroll
-  for (int v = 0; v < VPL; ++v)
-#pragma unroll
-    for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-  const int item = a.chunk_item[k];
-  const int node = a.node[item] & 0x7fffffff;
-  const float dv = (a.scale_mode == SCALE_DCOL_DROW) ? __ldg(a.mult + node) : 1.f;
-  gather_range<XT, VPL, V, fwd_in_flight<XT, YT, VPL, COMP, WIDE>(), OFF32>(
-      acc, static_cast<const XT*>(a.x), a.ldx, a.nvec, a.cent, a.cval, a.chunk_beg[k], a.chunk_end[k],
-      a.scale_mode, a.mult, dv, tl, TL, tmask);
-  float* prow = a.partial + (int64_t)k * a.ldp;
-#pragma unroll
-  for (int v = 0; v < VPL; ++v) {
-    const int vi = tl + v * TL;
-    if (vi < a.nvec) store_f32<V>(prow + vi * V, acc[v]);
-  }
-  __threadfence();
-  __syncwarp(tmask);
-  if (tl == 0) st_release(a.chunk_flag + k, epoch);
-}
-
-// out = gin_scale * X[node] + acc (one rounding) for the GIN form, else acc
-template <typename XT, int V>
-__device__ __forceinline__ void gin_self(const FwdArgs& a, int node, int vi, const float (&acc)[V], float (&out)[V]) {
-  if (a.gin) {
-    float xs[V];
-    Vec<XT, V>::load(static_cast<const XT*>(a.x) + (int64_t)node * a.ldx + (int64_t)vi * V, xs);
-#pragma unroll
-    for (int q = 0; q < V; ++q) out[q] = fmaf(a.gin_scale, xs[q], acc[q]);
-  } else {
-#pragma unroll
-    for (int q = 0; q < V; ++q) out[q] = acc[q];
-  }
+  return FORM == 2 || VPL > 4 ? 1 : VPL == 4 ? 2 : VPL == 1 && TLC == 32 ? 4 : 3;
 }
 
 // s + e == a + b exactly (Knuth's TwoSum; explicit roundings, no contraction)
@@ -410,146 +495,19 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
   e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bp)), __fsub_rn(b, bp));
 }
 
-template <typename XT, typename YT, int VPL, int V, bool COMP = false, bool WIDE = false, bool OFF32 = false>
-__device__ __forceinline__ void fwd_row(const FwdArgs& a, int item, unsigned epoch, int tl, int TL, unsigned tmask) {
-  float acc[VPL][V];
-#pragma unroll
-  for (int v = 0; v < VPL; ++v)
-#pragma unroll
-    for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-  const int nodew = a.node[item];
-  const int node = nodew & 0x7fffffff;
-  const bool internal = nodew < 0;
-  const bool need_dv = (a.scale_mode == SCALE_DCOL_DROW) || (a.prop_mode == PROP_RATIO);
-  const float dv = need_dv ? __ldg(a.mult + node) : 1.f;
-  const int c0 = a.chunk0[item];
-  if (c0 < 0) {
-    gather_range<XT, VPL, V, fwd_in_flight<XT, YT, VPL, COMP, WIDE>(), OFF32>(
-        acc, static_cast<const XT*>(a.x), a.ldx, a.nvec, a.ent, a.val, a.ptr[item], a.ptr[item + 1],
-        a.scale_mode, a.mult, dv, tl, TL, tmask);
-  } else {
-    for (int k = c0; k < a.n_chunks && a.chunk_item[k] == item; ++k) {
-      if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
-      const float* prow = a.partial + (int64_t)k * a.ldp;
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int vi = tl + v * TL;
-        if (vi < a.nvec) {
-          float t[V];
-          load_f32_cg<V>(prow + vi * V, t);
-#pragma unroll
-          for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], t[q]);
-        }
-      }
-    }
-  }
-  const int p = a.skip_parent ? -1 : a.par[item];
-  // compensated arithmetic for this row, a residual to read from the parent
-  const bool cmode = COMP && item >= a.comp_item0;
-  const bool cread = COMP && item >= a.comp_read0;
-  float cres[VPL][V];  // unused (and removed by the compiler) without COMP
-#pragma unroll
-  for (int v = 0; v < VPL; ++v)
-#pragma unroll
-    for (int q = 0; q < V; ++q) cres[v][q] = 0.f;
-  // after a failed (timed-out) wait the parent is left out; the error is recorded
-  if (p >= 0 && wait_flag(a.node_flag + p, epoch, a.qs, a.timeout_ns, (long long)node)) {
-    const float dp = (a.prop_mode == PROP_RATIO) ? __ldg(a.mult + p) : 1.f;
-    const int ps = a.par_slot[item];
-#pragma unroll
-    for (int v = 0; v < VPL; ++v) {
-      const int vi = tl + v * TL;
-      if (vi < a.nvec) {
-        float yp[V];
-        if (sizeof(YT) == 4 && !a.gin) {
-          load_y_cg<YT, V>(static_cast<const YT*>(a.y) + (int64_t)p * a.ldy + (int64_t)vi * V, yp);
-        } else {
-          load_f32_cg<V>(a.pstate + (int64_t)ps * a.ldp + vi * V, yp);
-        }
-        if (COMP && cmode) {
-          // parent value = yp + rp (rp: its residual); add with TwoSum and keep
-          // the rounding errors (of the ratio's product and quotient too)
-          float rp[V];
-          if (cread) {
-            load_f32_cg<V>(a.pcomp + (int64_t)ps * a.ldp + vi * V, rp);
-          } else {
-#pragma unroll
-            for (int q = 0; q < V; ++q) rp[q] = 0.f;
-          }
-#pragma unroll
-          for (int q = 0; q < V; ++q) {
-            float t = yp[q], r = rp[q];
-            if (a.prop_mode == PROP_RATIO) {
-              const float prod = __fmul_rn(yp[q], dv);
-              const float pe = fmaf(yp[q], dv, -prod);     // prod + pe == yp * dv
-              t = __fdiv_rn(prod, dp);
-              const float qe = __fdiv_rn(fmaf(-t, dp, prod), dp);  // t + qe ~ prod / dp
-              r = __fadd_rn(__fdiv_rn(fmaf(r, dv, pe), dp), qe);
-            }
-            float s_, e_;
-            two_sum(acc[v][q], t, s_, e_);
-            acc[v][q] = s_;
-            cres[v][q] = __fadd_rn(r, e_);
-          }
-        } else if (a.prop_mode == PROP_RATIO) {
-#pragma unroll
-          for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], __fdiv_rn(__fmul_rn(yp[q], dv), dp));
-        } else {
-#pragma unroll
-          for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], yp[q]);
-        }
-      }
-    }
-  }
-  if (COMP && cmode) {
-    // the row's value is acc + cres, rounded once; its residual is kept for
-    // the children of an internal node
-#pragma unroll
-    for (int v = 0; v < VPL; ++v)
-#pragma unroll
-      for (int q = 0; q < V; ++q) {
-        float s_, e_;
-        two_sum(acc[v][q], cres[v][q], s_, e_);
-        acc[v][q] = s_;
-        cres[v][q] = e_;
-      }
-    if (internal) {
-      float* crow = a.pcomp + (int64_t)a.self_slot[item] * a.ldp;
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int vi = tl + v * TL;
-        if (vi < a.nvec) store_f32<V>(crow + vi * V, cres[v]);
-      }
-    }
-  }
-  YT* yrow = static_cast<YT*>(a.y) + (int64_t)node * a.ldy;
-#pragma unroll
-  for (int v = 0; v < VPL; ++v) {
-    const int vi = tl + v * TL;
-    if (vi < a.nvec) {
-      float out[V];
-      gin_self<XT, V>(a, node, vi, acc[v], out);
-      store_vec<YT, V>(yrow + (int64_t)vi * V, out);
-    }
-  }
-  if (internal && !a.skip_parent) {
-    if (sizeof(YT) != 4 || a.gin) {
-      float* srow = a.pstate + (int64_t)a.self_slot[item] * a.ldp;
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int vi = tl + v * TL;
-        if (vi < a.nvec) store_f32<V>(srow + vi * V, acc[v]);
-      }
-    }
-    __threadfence();
-    __syncwarp(tmask);
-    if (tl == 0) st_release(a.node_flag + node, epoch);
-  }
-}
+// The register kernel hands out rows from kClaimQueues counters, one per warp
+// of a block: warp w of every block takes every kClaimQueues-th group.  Atomics
+// on one address complete one after another, about 0.9 ns apart on B200, which
+// alone cost 150 us of a 170,000-row product with one-row claims.  Each counter
+// is handed out in queue order and every block serves all of them, so the
+// progress argument of one queue holds.
+constexpr int kClaimQueues = kThreads / 32;
+constexpr int kClaimStride = 256;  // unsigned, 1 KiB: counters in separate L2 lines
 
 // The last block to finish resets the queue counters and, unless another pass
 // of the same product follows, publishes the launch epoch.
-__device__ __forceinline__ void finish_block(QueueState* qs, unsigned epoch, bool publish = true) {
+__device__ __forceinline__ void finish_block(QueueState* qs, unsigned epoch, bool publish = true,
+                                             unsigned* claims = nullptr) {
   __syncthreads();
   if (threadIdx.x == 0) {
     __threadfence();
@@ -558,52 +516,369 @@ __device__ __forceinline__ void finish_block(QueueState* qs, unsigned epoch, boo
       qs->next_chunk = 0;
       qs->next_row = 0;
       qs->done_blocks = 0;
+      for (int q = 0; claims && q < kClaimQueues; ++q) claims[q * kClaimStride] = 0;
       __threadfence();
       if (publish) atomicExch(&qs->epoch, epoch);
     }
   }
 }
 
-template <typename XT, typename YT, int VPL, int V, bool COMP = false, bool WIDE = false, bool OFF32 = false>
-__global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, COMP, WIDE>()))
-    fwd_kernel(const FwdArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int TL = a.team;
-  const int team = lane / TL;
-  const int tl = lane & (TL - 1);
-  const int teams = 32 / TL;
-  const unsigned tmask = (TL == 32) ? 0xffffffffu : (((1u << TL) - 1u) << (team * TL));
-  const unsigned epoch = *(volatile unsigned*)&a.qs->epoch + 1u;
+// ---- register kernel ------------------------------------------------------------
+// Short rows on an operand that L2 holds are bound by latency: a row is a chain
+// of dependent loads (claim, record, entries, gathers, parent's flag, parent's
+// row).  Each warp therefore runs its rows as a pipeline: while the gathers of
+// row i are in flight, row i + 1's entries load and its parent's flag is
+// acquired, and the claim and the record of the row after that are made; the
+// parent's row of row i + 1 is then fetched together with its gathers.
+//
+// Teams that share a warp (rows narrower than 32 vectors) step together.  A
+// wait then holds up the whole warp, which is safe as long as what it waits
+// for is not the warp's own: an item whose parent lies fewer than 32 queue
+// positions before it carries kNearBit, and a group of items with one runs its
+// row ends team by team, in queue order.
+//
+// Progress: a warp finishes its groups in the order it claimed them, also with
+// the next claim already made, and an item depends on earlier items only.
+// Record of an item: x = node | kNearBit | internal << 31, y = parent node or
+// -1, z = first entry and w = entries of the row; a split row has its first
+// chunk and minus the number of chunks there, a presummed row its place among
+// the presummed rows and kPreMark.
+//
+// Measured on B200 against one row per claim and warp with every load in turn
+// (bit-identical): 170,000-node GCN graph, 128 FP32 columns 262 -> 163 us, 128
+// BF16 210 -> 146, 40 BF16 174 -> 116; 100,000 nodes, 47 FP32 columns (no
+// 16-byte vectors) 273 -> 104, GIN with 64 columns 122 -> 79.  What is left is
+// instruction issue and the exposed round trip per row, not bandwidth: no
+// gather at all leaves 66 us of the first (profiled by leaving parts out).
+constexpr int kNearBit = 0x40000000;
+constexpr int kNodeMask = 0x3fffffff;
+// null records past the last item: a group there starts at item n at most
+constexpr int kMetaPad = 32;
+// entry count of a presummed row's record
+constexpr int kPreMark = INT_MIN;
 
-  if (a.n_chunks > 0) {
+// What a register-kernel instantiation leaves out: FORM_PLAIN has no GIN term
+// and no compensation.
+enum RowForm : int { FORM_PLAIN = 0, FORM_GIN = 1, FORM_COMP = 2 };
+
+template <typename XT, typename YT, int VPL, int V, int FORM, int TLC>
+__global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, TLC>())) fwd_kernel(const FwdArgs a) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr bool COMP = FORM == FORM_COMP;
+  // parents' rows come from the FP32 state rows
+  const bool state = sizeof(YT) != 4 || FORM == FORM_GIN || (COMP && a.gin);
+  const int lane = threadIdx.x & 31;
+  const int TL = TLC ? TLC : a.team;
+  const int tl = lane & (TL - 1);
+  const int team = lane / TL;
+  const unsigned teams = 32 / TL;
+  const unsigned epoch = *(volatile unsigned*)&a.qs->epoch + 1u;
+  const Lane<XT, VPL, V, TLC != 32> ln(a.x, a.ldx, a.nvec, tl, TL);
+  const bool drow = a.scale_mode == SCALE_DCOL_DROW;
+  const bool ratio = a.prop_mode == PROP_RATIO;
+  const float* vals = a.scale_mode == SCALE_SIGN ? nullptr : a.scale_mode == SCALE_VALUES ? a.val : a.sval;
+  const unsigned n = (unsigned)a.n_items;
+
+  // ---- sums that wait on nothing: chunks of split rows, then the presummed
+  // rows; one per team and claim, the next claim made ahead
+  const unsigned n_split = (unsigned)a.n_chunks;
+  const unsigned n_sums = n_split + (unsigned)a.n_pre;
+  if (n_sums > 0) {
+    const float* cvals = a.scale_mode == SCALE_SIGN ? nullptr : a.scale_mode == SCALE_VALUES ? a.cval : a.csval;
+    unsigned pend = 0;
+    if (lane == 0) pend = atomicAdd(&a.qs->next_chunk, teams);
     for (;;) {
-      unsigned base = 0;
-      if (lane == 0) base = atomicAdd(&a.qs->next_chunk, (unsigned)teams);
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (base >= (unsigned)a.n_chunks) break;
+      const unsigned base = __shfl_sync(kAll, pend, 0);
+      if (base >= n_sums) break;
+      if (lane == 0) pend = atomicAdd(&a.qs->next_chunk, teams);
       const unsigned k = base + team;
-      if (k < (unsigned)a.n_chunks) fwd_chunk<XT, YT, VPL, V, COMP, WIDE, OFF32>(a, (int)k, epoch, tl, TL, tmask);
+      const bool have = k < n_sums;
+      const bool split = k < n_split;
+      const uint32_t* ent = a.ent;
+      const float* cv = vals;
+      float* out = nullptr;
+      int len = 0, node = 0;
+      if (have) {
+        if (split) {
+          const int64_t cb = a.chunk_beg[k];
+          len = (int)(a.chunk_end[k] - cb);
+          node = a.node[a.chunk_item[k]] & 0x7fffffff;
+          ent = a.cent + cb;
+          cv = cvals ? cvals + cb : nullptr;
+          out = a.partial + (int64_t)k * a.ldp;
+        } else {
+          const int4 r = __ldg(a.pre + (k - n_split));
+          len = r.w;
+          node = r.y;
+          ent = a.ent + (uint32_t)r.z;
+          if (vals) cv = vals + (uint32_t)r.z;
+          out = a.pre_rows ? a.pre_rows + (int64_t)(k - n_split) * a.ldp
+                           : static_cast<float*>(a.y) + row_off(node, a.ldy);
+        }
+      }
+      uint32_t e = 0;
+      float s = 0.f;
+      if (tl < len) {
+        e = __ldg(ent + tl);
+        s = reg_scale(e, cv, tl, a.scale_mode, a.mult);
+      }
+      const float dv = drow ? __ldg(a.mult + node) : 1.f;
+      float acc[VPL][V];
+#pragma unroll
+      for (int v = 0; v < VPL; ++v)
+#pragma unroll
+        for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
+      gather_row<XT, VPL, V, TLC>(acc, ln, ent, cv, len, TLC == 32 ? len : __reduce_max_sync(kAll, len), e, s, dv,
+                                  a.scale_mode, a.mult, tl, TL, [] {});
+      if (have) {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          const int vi = tl + v * TL;
+          if (vi < a.nvec) store_f32<V>(out + vi * V, acc[v]);
+        }
+      }
+      // the barrier orders the team's stores before its first lane's release,
+      // which carries them (cumulativity)
       __syncwarp();
+      if (have && tl == 0) st_release(a.chunk_flag + k, epoch);
     }
   }
-  // claims of rows_per_claim rows per team while the queue is in level 0, of
-  // rows_per_claim_deep below it (sized by where the warp's last claim fell)
-  unsigned last = 0;
-  for (;;) {
-    const int R = last < (unsigned)a.n_root ? a.rows_per_claim : a.rows_per_claim_deep;
-    unsigned base = 0;
-    if (lane == 0) base = atomicAdd(&a.qs->next_row, (unsigned)(teams * R));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= (unsigned)a.n_items) break;
-    last = base;
-    for (int r = 0; r < R; ++r) {
-      const unsigned item = base + team + (unsigned)(r * teams);
-      if (item >= (unsigned)a.n_items) break;
-      fwd_row<XT, YT, VPL, V, COMP, WIDE, OFF32>(a, (int)item, epoch, tl, TL, tmask);
+
+  // ---- rows: one group of `teams` items per claim from the warp's queue, the
+  // next claim made ahead
+  const unsigned wq = threadIdx.x >> 5;
+  unsigned pend = 0;
+  if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+  // first item of the warp's next group; n when the queue is exhausted
+  auto next_group = [&]() -> unsigned {
+    const unsigned g = (__shfl_sync(kAll, pend, 0) * kClaimQueues + wq) * teams;
+    if (g >= n) return n;  // the claim stays pending: every later call ends here too
+    if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+    return g;
+  };
+  unsigned g0 = next_group();
+  if (g0 < n) {
+    unsigned g1 = next_group();
+    int4 m0 = __ldg(a.meta + g0 + team), m1 = __ldg(a.meta + g1 + team);
+    uint32_t e0 = 0;
+    float s0 = 0.f;
+    unsigned f0 = 0;
+    if (tl < m0.w) {
+      e0 = __ldg(a.ent + (uint32_t)m0.z + tl);
+      s0 = reg_scale(e0, vals ? vals + (uint32_t)m0.z : nullptr, tl, a.scale_mode, a.mult);
     }
-    __syncwarp();
+    if (a.skip_parent) m0.y = -1, m1.y = -1;
+    if (m0.y >= 0) f0 = ld_acquire(a.node_flag + m0.y);
+    while (g0 < n) {
+      const unsigned item = g0 + team;
+      const bool have = TLC == 32 || item < n;
+      const int node = m0.x & kNodeMask;
+      const int p = m0.y;
+      const float dv = drow || ratio ? __ldg(a.mult + node) : 1.f;
+      // the parent's row, if that is final already
+      const bool ready = p >= 0 && f0 == epoch;
+      float yp[VPL][V];
+      float dp = 1.f;
+      auto load_parent = [&]() {
+        const float* src;
+        if (state) {
+          src = a.pstate + (int64_t)__ldg(a.par_slot + item) * a.ldp;
+        } else {
+          src = static_cast<const float*>(a.y) + row_off(p, a.ldy);
+        }
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          const int vi = tl + v * TL;
+          if (vi < a.nvec) load_f32_cg<V>(src + (int64_t)vi * V, yp[v]);
+        }
+      };
+      if (ready) load_parent();
+      typename Raw<XT, V>::type xself[VPL];  // GIN: the row's own X, for its store
+      auto load_self = [&]() {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          xself[v] = Raw<XT, V>::zero();
+          if (a.gin && have) xself[v] = Raw<XT, V>::load(reinterpret_cast<const XT*>(ln.row(node) + ln.off[v]));
+        }
+      };
+      // ahead of the gathers, but for one piece per lane, where those registers
+      // are worth more as occupancy (100,000-node GIN, 256 FP32 columns: 198 ->
+      // 178 us; 200,000 nodes, 128 columns: 376 -> 353 us the other way)
+      if (FORM != FORM_PLAIN && VPL > 1) load_self();
+      if (ratio && p >= 0) dp = __ldg(a.mult + p);
+      float acc[VPL][V];
+#pragma unroll
+      for (int v = 0; v < VPL; ++v)
+#pragma unroll
+        for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
+      const int len = m0.w > 0 ? m0.w : 0;
+      uint32_t e1 = 0;
+      float s1 = 0.f;
+      unsigned f1 = 0;
+      gather_row<XT, VPL, V, TLC>(acc, ln, a.ent + (uint32_t)m0.z, vals ? vals + (uint32_t)m0.z : nullptr, len,
+                                  TLC == 32 ? len : __reduce_max_sync(kAll, len), e0, s0, drow ? dv : 1.f,
+                                  a.scale_mode, a.mult, tl, TL, [&] {
+                                    if (tl < m1.w) {
+                                      e1 = __ldg(a.ent + (uint32_t)m1.z + tl);
+                                      if (vals) s1 = __ldg(vals + (uint32_t)m1.z + tl);
+                                    }
+                                    if (m1.y >= 0) f1 = ld_acquire(a.node_flag + m1.y);
+                                  });
+
+      if (FORM != FORM_PLAIN && VPL == 1) load_self();
+
+      // ---- the row's end: chunk partials, parent, store, ready flag
+      const int serial = TLC != 32 && __any_sync(kAll, have && (m0.x & kNearBit) != 0) ? (int)teams : 1;
+      for (int t = 0; t < serial; ++t) {
+        if (have && (serial == 1 || team == t)) {
+          if (m0.w == kPreMark) {
+            // summed ahead: record z is its place among the presummed rows
+            if (wait_flag(a.chunk_flag + n_split + m0.z, epoch, a.qs, a.timeout_ns, (long long)m0.z)) {
+              const float* prow = a.pre_rows ? a.pre_rows + (int64_t)m0.z * a.ldp
+                                             : static_cast<const float*>(a.y) + row_off(node, a.ldy);
+#pragma unroll
+              for (int v = 0; v < VPL; ++v) {
+                const int vi = tl + v * TL;
+                if (vi < a.nvec) load_f32_cg<V>(prow + vi * V, acc[v]);
+              }
+            }
+          }
+          for (int k = m0.z, ke = m0.z - m0.w; k < ke && m0.w < 0 && m0.w != kPreMark; ++k) {
+            if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
+            const float* prow = a.partial + (int64_t)k * a.ldp;
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) {
+              const int vi = tl + v * TL;
+              if (vi < a.nvec) {
+                float part[V];
+                load_f32_cg<V>(prow + vi * V, part);
+#pragma unroll
+                for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], part[q]);
+              }
+            }
+          }
+          // compensated arithmetic for this row, a residual to read from the parent
+          const bool cmode = COMP && (int)item >= a.comp_item0;
+          const bool cread = COMP && (int)item >= a.comp_read0;
+          float cres[VPL][V];  // unused (and removed by the compiler) without COMP
+#pragma unroll
+          for (int v = 0; v < VPL; ++v)
+#pragma unroll
+            for (int q = 0; q < V; ++q) cres[v][q] = 0.f;
+          // after a failed (timed-out) wait the parent is left out; the error is recorded
+          bool add = ready;
+          if (p >= 0 && !ready && wait_flag(a.node_flag + p, epoch, a.qs, a.timeout_ns, (long long)node)) {
+            load_parent();
+            add = true;
+          }
+          if (add) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) {
+              const int vi = tl + v * TL;
+              if (vi < a.nvec) {
+                if (COMP && cmode) {
+                  // parent value = yp + rp (rp: its residual); add with TwoSum and keep
+                  // the rounding errors (of the ratio's product and quotient too)
+                  float rp[V];
+                  if (cread) {
+                    load_f32_cg<V>(a.pcomp + (int64_t)__ldg(a.par_slot + item) * a.ldp + vi * V, rp);
+                  } else {
+#pragma unroll
+                    for (int q = 0; q < V; ++q) rp[q] = 0.f;
+                  }
+#pragma unroll
+                  for (int q = 0; q < V; ++q) {
+                    float y = yp[v][q], r = rp[q];
+                    if (ratio) {
+                      const float prod = __fmul_rn(yp[v][q], dv);
+                      const float pe = fmaf(yp[v][q], dv, -prod);  // prod + pe == yp * dv
+                      y = __fdiv_rn(prod, dp);
+                      const float qe = __fdiv_rn(fmaf(-y, dp, prod), dp);  // y + qe ~ prod / dp
+                      r = __fadd_rn(__fdiv_rn(fmaf(r, dv, pe), dp), qe);
+                    }
+                    float s_, e_;
+                    two_sum(acc[v][q], y, s_, e_);
+                    acc[v][q] = s_;
+                    cres[v][q] = __fadd_rn(r, e_);
+                  }
+                } else if (ratio) {
+#pragma unroll
+                  for (int q = 0; q < V; ++q)
+                    acc[v][q] = __fadd_rn(acc[v][q], __fdiv_rn(__fmul_rn(yp[v][q], dv), dp));
+                } else {
+#pragma unroll
+                  for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], yp[v][q]);
+                }
+              }
+            }
+          }
+          const bool keep = m0.x < 0 && !a.skip_parent;  // children read this row
+          const int ss = keep && (state || COMP) ? __ldg(a.self_slot + item) : 0;
+          if (COMP && cmode) {
+            // the row's value is acc + cres, rounded once; its residual is kept for
+            // the children of an internal node
+#pragma unroll
+            for (int v = 0; v < VPL; ++v)
+#pragma unroll
+              for (int q = 0; q < V; ++q) {
+                float s_, e_;
+                two_sum(acc[v][q], cres[v][q], s_, e_);
+                acc[v][q] = s_;
+                cres[v][q] = e_;
+              }
+            if (keep) {
+              float* crow = a.pcomp + (int64_t)ss * a.ldp;
+#pragma unroll
+              for (int v = 0; v < VPL; ++v) {
+                const int vi = tl + v * TL;
+                if (vi < a.nvec) store_f32<V>(crow + vi * V, cres[v]);
+              }
+            }
+          }
+          YT* yrow = static_cast<YT*>(a.y) + row_off(node, a.ldy);
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) {
+            const int vi = tl + v * TL;
+            if (vi < a.nvec) {
+              if constexpr (FORM == FORM_PLAIN) {
+                store_vec<YT, V>(yrow + (int64_t)vi * V, acc[v]);
+              } else {
+                float xs[V], out[V];
+                Raw<XT, V>::widen(xself[v], xs);
+#pragma unroll
+                for (int q = 0; q < V; ++q) out[q] = a.gin ? fmaf(a.gin_scale, xs[q], acc[v][q]) : acc[v][q];
+                store_vec<YT, V>(yrow + (int64_t)vi * V, out);
+              }
+            }
+          }
+          if (keep) {
+            if (state) {
+              float* srow = a.pstate + (int64_t)ss * a.ldp;
+#pragma unroll
+              for (int v = 0; v < VPL; ++v) {
+                const int vi = tl + v * TL;
+                if (vi < a.nvec) store_f32<V>(srow + vi * V, acc[v]);
+              }
+            }
+            // as for the chunks: the team's stores before its first lane's release
+            __syncwarp(TLC == 32 || TL == 32 ? kAll : (((1u << TL) - 1u) << (team * TL)));
+            if (tl == 0) st_release(a.node_flag + node, epoch);
+          }
+        }
+        __syncwarp();
+      }
+      // ---- on to the next row: its entries are here, the record behind it loads
+      g0 = g1;
+      m0 = m1;
+      e0 = e1;
+      s0 = vals ? s1 : tl < m0.w ? reg_scale(e0, nullptr, 0, a.scale_mode, a.mult) : 0.f;
+      f0 = f1;
+      g1 = next_group();
+      m1 = __ldg(a.meta + g1 + team);
+      if (a.skip_parent) m1.y = -1;
+    }
   }
-  finish_block(a.qs, epoch, a.publish_epoch != 0);
+  finish_block(a.qs, epoch, a.publish_epoch != 0, a.claims);
 }
 
 // ============================================================================

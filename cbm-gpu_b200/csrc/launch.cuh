@@ -43,18 +43,14 @@ int cached_grid(GridCache& c, K kernel, int device, int block, int smem) {
   return g;
 }
 
-template <typename XT, typename YT, int VPL, int V, bool COMP = false, bool WIDE = false>
+template <typename XT, typename YT, int VPL, int V, int FORM>
 int launch_fwd_t(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
+  // full-warp teams have their own instantiation (also where X's rows lie 2^32
+  // bytes apart or more: that one has 32-bit row strides)
   static GridCache cache[2];
-  // BF16 X with fewer than 2^32 elements takes 32-bit row offsets (measured
-  // faster there; FP32 X keeps the widening multiply)
-  bool off32 = false;
-  auto kern = fwd_kernel<XT, YT, VPL, V, COMP, WIDE, false>;
-  if constexpr (sizeof(XT) == 2) {
-    off32 = (uint64_t)P->n_cols * (uint64_t)a.ldx <= 0xffffffffull;
-    if (off32) kern = fwd_kernel<XT, YT, VPL, V, COMP, WIDE, true>;
-  }
-  const int grid = cached_grid(cache[off32 ? 1 : 0], kern, P->device, kThreads, 0);
+  const bool full = a.team == 32 && (uint64_t)a.ldx * sizeof(XT) <= 0xffffffffull;
+  auto kern = full ? fwd_kernel<XT, YT, VPL, V, FORM, 32> : fwd_kernel<XT, YT, VPL, V, FORM, 0>;
+  const int grid = cached_grid(cache[full ? 1 : 0], kern, P->device, kThreads, 0);
   if (grid <= 0) return CBM_ERR_CUDA;
   kern<<<grid, kThreads, 0, st>>>(a);
   P->launches++;
@@ -135,13 +131,13 @@ int launch_tma_any(cbm_plan* P, const FwdArgs& a, int team, int vpl, const CUten
   return CBM_ERR_INTERNAL;
 }
 
-template <typename XT, typename YT, int V, bool COMP = false>
+template <typename XT, typename YT, int V, int FORM>
 int launch_fwd_v(cbm_plan* P, const FwdArgs& a, int vpl, cudaStream_t st) {
   switch (vpl) {
-    case 1: return launch_fwd_t<XT, YT, 1, V, COMP>(P, a, st);
-    case 2: return launch_fwd_t<XT, YT, 2, V, COMP>(P, a, st);
-    case 4: return launch_fwd_t<XT, YT, 4, V, COMP>(P, a, st);
-    default: return launch_fwd_t<XT, YT, 8, V, COMP>(P, a, st);
+    case 1: return launch_fwd_t<XT, YT, 1, V, FORM>(P, a, st);
+    case 2: return launch_fwd_t<XT, YT, 2, V, FORM>(P, a, st);
+    case 4: return launch_fwd_t<XT, YT, 4, V, FORM>(P, a, st);
+    default: return launch_fwd_t<XT, YT, 8, V, FORM>(P, a, st);
   }
 }
 
@@ -185,9 +181,7 @@ int launch_staged_bf16_bf16(cbm_plan* P, const FwdArgs& a, int team, int vpl, cu
 int launch_tma(cbm_plan* P, const FwdArgs& a, int32_t xdt, int32_t ydt, int team, int vpl, const CUtensorMap& map,
                cudaStream_t st);
 int launch_fwd_f32(cbm_plan* P, const FwdArgs& a, bool vec, int vpl, cudaStream_t st);
-// wide: on trees where few rows wait on a parent, one-vector rows of BF16 X
-// and FP32 Y take the 4-block instantiation (fwd_min_blocks)
-int launch_fwd_bf16(cbm_plan* P, const FwdArgs& a, int32_t ydt, bool vec, int vpl, bool wide, cudaStream_t st);
+int launch_fwd_bf16(cbm_plan* P, const FwdArgs& a, int32_t ydt, bool vec, int vpl, cudaStream_t st);
 // compensated propagation: BF16 X only (the precision form), register kernel
 int launch_fwd_comp(cbm_plan* P, const FwdArgs& a, int32_t ydt, bool vec, int vpl, cudaStream_t st);
 // second pass of a two-pass product (FP32 Y)

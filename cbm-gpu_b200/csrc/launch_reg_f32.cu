@@ -3,17 +3,22 @@
 #include "launch.cuh"
 
 namespace cbm {
+template <int FORM>
+int launch_f32_form(cbm_plan* P, const FwdArgs& a, bool vec, int vpl, cudaStream_t st) {
+  return vec ? launch_fwd_v<float, float, 4, FORM>(P, a, vpl, st) : launch_fwd_v<float, float, 1, FORM>(P, a, vpl, st);
+}
+
 int launch_fwd_f32(cbm_plan* P, const FwdArgs& a, bool vec, int vpl, cudaStream_t st) {
-  return vec ? launch_fwd_v<float, float, 4>(P, a, vpl, st) : launch_fwd_v<float, float, 1>(P, a, vpl, st);
+  return a.gin ? launch_f32_form<FORM_GIN>(P, a, vec, vpl, st) : launch_f32_form<FORM_PLAIN>(P, a, vec, vpl, st);
 }
 
 int launch_fwd_comp(cbm_plan* P, const FwdArgs& a, int32_t ydt, bool vec, int vpl, cudaStream_t st) {
   if (ydt == CBM_F32) {
-    return vec ? launch_fwd_v<__nv_bfloat16, float, 8, true>(P, a, vpl, st)
-               : launch_fwd_v<__nv_bfloat16, float, 1, true>(P, a, vpl, st);
+    return vec ? launch_fwd_v<__nv_bfloat16, float, 8, FORM_COMP>(P, a, vpl, st)
+               : launch_fwd_v<__nv_bfloat16, float, 1, FORM_COMP>(P, a, vpl, st);
   }
-  return vec ? launch_fwd_v<__nv_bfloat16, __nv_bfloat16, 8, true>(P, a, vpl, st)
-             : launch_fwd_v<__nv_bfloat16, __nv_bfloat16, 1, true>(P, a, vpl, st);
+  return vec ? launch_fwd_v<__nv_bfloat16, __nv_bfloat16, 8, FORM_COMP>(P, a, vpl, st)
+             : launch_fwd_v<__nv_bfloat16, __nv_bfloat16, 1, FORM_COMP>(P, a, vpl, st);
 }
 
 int launch_prop(cbm_plan* P, const PropArgs& a, bool vec, int vpl, cudaStream_t st) {

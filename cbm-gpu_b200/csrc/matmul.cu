@@ -157,10 +157,9 @@ bool tma_shape(int64_t nvec, int v, int team, int vpl) {
   return nvec >= 8 && (nvec & (nvec - 1)) == 0 && nvec == (int64_t)team * vpl && nvec * v <= 256 && vpl <= 2;
 }
 
-int launch_fwd(cbm_plan* P, const FwdArgs& a, int32_t xdt, int32_t ydt, bool vec, int vpl, bool shallow,
-               cudaStream_t st) {
+int launch_fwd(cbm_plan* P, const FwdArgs& a, int32_t xdt, int32_t ydt, bool vec, int vpl, cudaStream_t st) {
   if (xdt == CBM_F32) return launch_fwd_f32(P, a, vec, vpl, st);
-  return launch_fwd_bf16(P, a, ydt, vec, vpl, shallow, st);
+  return launch_fwd_bf16(P, a, ydt, vec, vpl, st);
 }
 
 template <typename T>
@@ -327,8 +326,9 @@ int64_t cbm_plan_workspace_bytes(const cbm_plan* P, int32_t op, int64_t n_cols, 
     const int64_t t_chunks = P->adj_built ? P->n_t_chunks : (2 * P->nnz / P->chunk_nnz + 1);
     rows = P->n_internal + t_chunks + (P->adj_built ? P->n_rev_chunks : P->n_internal);
   } else {
-    rows = P->n_chunks + ((y_dtype == CBM_BF16 || op == CBM_OP_GIN) ? P->n_internal : 0) +
-           (comp_active(P, x_dtype) ? P->n_internal : 0);
+    // presummed rows need room only where Y cannot hold their FP32 sums
+    const bool state = y_dtype == CBM_BF16 || op == CBM_OP_GIN;
+    rows = P->n_chunks + (state ? P->n_internal + P->n_pre : 0) + (comp_active(P, x_dtype) ? P->n_internal : 0);
   }
   return align256(rows * ldp * 4) + 256;
 }
@@ -364,6 +364,13 @@ int cbm_plan_debug_set_parent(cbm_plan* P, int64_t item, int32_t parent_node, vo
   int32_t par_item = -1;
   for (int64_t i = 0; parent_node >= 0 && i < P->n_items; ++i)
     if (P->h_order[i] == parent_node) par_item = (int32_t)i;
+  // the item's record too: its node word (near bit) and parent
+  P->h_item_par[item] = parent_node;
+  P->h_item_par_item[item] = par_item;
+  const int32_t rec[2] = {record_node(P, item), parent_node};
+  if (cudaMemcpyAsync(reinterpret_cast<char*>(P->d_meta + item), rec, sizeof(rec), cudaMemcpyHostToDevice, st) !=
+      cudaSuccess)
+    return CBM_ERR_CUDA;
   if (cudaMemcpyAsync(P->d_par_item + item, &par_item, sizeof(int32_t), cudaMemcpyHostToDevice, st) != cudaSuccess)
     return CBM_ERR_CUDA;
   return cuda_status(cudaStreamSynchronize(st));
@@ -434,6 +441,9 @@ int matmul_impl(cbm_plan* P, int32_t op, float gin_scale, const void* x, int32_t
     FwdArgs a;
     std::memset(&a, 0, sizeof(a));
     a.n_items = (int32_t)P->n_items;
+    a.meta = P->d_meta;
+    a.sval = P->d_sval;
+    a.csval = P->d_csval;
     a.node = P->d_node;
     a.ptr = P->d_ptr;
     a.ent = P->d_ent;
@@ -461,12 +471,16 @@ int matmul_impl(cbm_plan* P, int32_t op, float gin_scale, const void* x, int32_t
     a.ldp = (int32_t)ldp;
     a.partial = static_cast<float*>(ws);
     a.pstate = ws ? static_cast<float*>(ws) + P->n_chunks * ldp : nullptr;
+    a.n_pre = (int32_t)P->n_pre;
+    a.pre = P->d_pre;
+    a.claims = P->d_claims;
     a.gin = gin ? 1 : 0;
     a.gin_scale = gin_scale;
     a.comp_item0 = (int32_t)P->n_items;
     a.comp_read0 = (int32_t)P->n_items;
+    if (state_rows && P->n_pre > 0) a.pre_rows = a.pstate + P->n_internal * ldp;
     if (comp) {
-      a.pcomp = static_cast<float*>(ws) + (P->n_chunks + (state_rows ? P->n_internal : 0)) * ldp;
+      a.pcomp = static_cast<float*>(ws) + (P->n_chunks + (state_rows ? P->n_internal + P->n_pre : 0)) * ldp;
       a.comp_item0 = (int32_t)P->level_start[P->comp_depth];
       a.comp_read0 = (int32_t)P->level_start[std::min<int64_t>(P->comp_depth + 1, P->levels)];
     }
@@ -482,17 +496,18 @@ int matmul_impl(cbm_plan* P, int32_t op, float gin_scale, const void* x, int32_t
     a.timeout_ns = P->timeout_ns;
     a.publish_epoch = 1;
     int s_team = 0, s_vpl = 0;
+    // AUTO takes the register kernel for rows of at most 32 vectors and on deep
+    // trees, the staged kernel for wider rows on shallow trees.  Measured on
+    // B200 (staged -> register, us): 800,000 nodes in 48 graphs, 64 BF16
+    // columns 944 -> 452; 200,000-node power-law graph, 32 / 64 / 128 FP32
+    // columns 397 / 380 / 313 -> 172 / 205 / 295; 1M nodes, 64 / 128 FP32
+    // columns 1332 / 1476 -> 936 / 1429; 400,000 nodes of mean degree 50, 128
+    // BF16 columns 1308 -> 1202.  256 FP32 columns: shallow 213 -> 297 and,
+    // with 1M nodes, 1943 -> 2702, deep (100,000 nodes, 84 % of the rows below
+    // level 0) 194 -> 167; 512 columns, deep 234 -> 180.
     // The GIN form runs on the register kernel (its self term and state rows
-    // stay out of the staged kernel's registers).  So does AUTO on trees where
-    // most rows wait on a parent: there the work is a chain of short waits,
-    // and the register kernel's lighter rows finish them sooner (measured on
-    // the 170K-node GCN graph, 84 % of rows below level 0: 0.30 -> 0.18 ms at
-    // 40 FP32 columns, 0.35 -> 0.23 ms at 128 BF16 columns; the 1M-node and
-    // 2.4M-node power-law graphs, 5 % and 40 % below level 0, keep the staged
-    // kernel).
-    // (rows of at most 512 bytes: the widths measured; wider rows keep the
-    // staged kernel, whose ring carries more bytes in flight per lane)
-    const bool deep_tree = (P->n_items - P->n_root) * 2 > P->n_items && cols * elem_size(xdt) <= 512;
+    // stay out of the staged kernel's registers).
+    const bool narrow = nvec <= 32 || P->deep;
     // Two passes (FP32 Y, no GIN term, no compensation): every row's delta sum
     // first, with no parent waits, then the parent terms in level order
     // (prop_kernel).  Opt-in: AUTO keeps the fused pass, which measured as
@@ -510,7 +525,7 @@ int matmul_impl(cbm_plan* P, int32_t op, float gin_scale, const void* x, int32_t
       a.n_units = 0;
     }
     const bool staged = sh.vec && !gin && P->variant != CBM_VARIANT_REGISTER &&
-                        !(P->variant == CBM_VARIANT_AUTO && deep_tree && !two_pass) &&
+                        !(P->variant == CBM_VARIANT_AUTO && narrow) &&
                         staged_shape(nvec, sh.v, P->staged_team, &s_team, &s_vpl);
     const bool tma = staged && P->variant == CBM_VARIANT_TMA && tma_shape(nvec, sh.v, s_team, s_vpl);
     int rc;
@@ -526,11 +541,16 @@ int matmul_impl(cbm_plan* P, int32_t op, float gin_scale, const void* x, int32_t
       a.team = s_team;
       rc = launch_staged(P, a, xdt, ydt, s_team, s_vpl, st);
     } else {
-      // on such trees level-0 claims of two rows also serve narrow operands
-      // better (40 BF16 columns on the GCN graph: 0.26 -> 0.17 ms)
-      if (P->variant == CBM_VARIANT_AUTO && deep_tree && !two_pass)
-        a.rows_per_claim = std::min<int32_t>(a.rows_per_claim, 2);
-      rc = launch_fwd(P, a, xdt, ydt, sh.vec, vpl, !deep_tree || two_pass, st);
+      // on deep trees, whose levels are in length order, two rows of 32 FP32
+      // vectors share a warp (170,000-node GCN graph, 128 columns: 193 -> 163
+      // us; unsorted rows leave one of the two idle: 295 -> 385 on a shallow
+      // tree)
+      if (sh.v == 4 && team == 32 && vpl == 1 && P->deep) {
+        team = 16;
+        vpl = 2;
+        a.team = team;
+      }
+      rc = launch_fwd(P, a, xdt, ydt, sh.vec, vpl, st);
     }
     if (rc) return rc;
     if (two_pass) {

@@ -49,8 +49,14 @@ struct cbm_plan {
   std::vector<uint32_t> h_ent;    // column | sign << 31, item order
   std::vector<float> h_val;       // values in item order (empty when all are +-1)
 
+  std::vector<int32_t> h_item_par;       // parent node per item, as on the device
+  std::vector<int32_t> h_item_par_item;  // its queue position, -1
+
   // forward layout (device); d_ptr/d_ent/d_val and d_cent/d_cval are the
   // stream layout rebuilt with the chunk size (build_layout)
+  int4* d_meta = nullptr;       // one 16-byte record per item (kernels.cuh, item_meta)
+  float* d_sval = nullptr;      // s * m[col] per entry of d_ent / d_cent, once the plan has
+  float* d_csval = nullptr;     // multipliers (square A, values +-1; null: formed in the kernel)
   int32_t* d_node = nullptr;
   int64_t* d_ptr = nullptr;
   uint32_t* d_ent = nullptr;
@@ -66,6 +72,14 @@ struct cbm_plan {
   cbm::QueueState* d_qs = nullptr;
   // forward chunks
   int64_t n_chunks = 0, long_rows = 0;
+  // presummed rows (register kernel, deep trees): long rows below level 0 whose
+  // sums are formed before the rows that wait on parents
+  bool deep = false;              // most rows hang below level 0
+  std::vector<char> pre_row;      // per item: summed ahead (unless split)
+  int64_t n_pre = 0;
+  int4* d_pre = nullptr;
+  unsigned* d_claims = nullptr;   // the register kernel's row counters
+  int64_t n_ent = 0, n_cent = 0;  // entries of d_ent and d_cent
   int32_t* d_chunk0 = nullptr;
   int32_t* d_chunk_item = nullptr;
   int64_t* d_chunk_beg = nullptr;
@@ -126,6 +140,8 @@ namespace cbm {
 int cuda_status(cudaError_t e);
 void free_all(std::vector<void*>& v);
 int build_layout(cbm_plan* P, cudaStream_t st);
+int scale_entries(cbm_plan* P, cudaStream_t st);
+int32_t record_node(const cbm_plan* P, int64_t item);
 int build_units(cbm_plan* P, cudaStream_t st);
 int32_t claim_rows(const cbm_plan* P);
 int32_t deep_rows_per_claim(const cbm_plan* P);

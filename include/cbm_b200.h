@@ -151,10 +151,11 @@ int cbm_plan_set_multipliers(cbm_plan* plan, const float* d_multipliers, void* s
 
 /* Tuning knobs.  chunk_nnz (>= 32): rows with more entries are summed in
  * chunks of that size by separate teams (host-side re-layout + upload).
- * rows_per_claim (>= 1): consecutive level-0 rows a team takes per queue
- * claim; rows_per_claim_deep (>= 0): the same for rows below level 0, which
- * wait on their parents (0: automatic, one row when more than a quarter of the
- * rows are below level 0, else rows_per_claim).
+ * rows_per_claim (>= 1): consecutive level-0 rows a team of the staged kernel
+ * takes per queue claim; rows_per_claim_deep (>= 0): the same for rows below
+ * level 0, which wait on their parents (0: automatic, one row when more than a
+ * quarter of the rows are below level 0, else rows_per_claim).  The register
+ * kernel claims one row per team.
  * variant: which forward kernel runs on the 16-byte vector path.
  * hot_rows (>= 0): the staged kernel asks L2 to keep the X rows of this many
  * most-gathered columns and to evict the others and the output rows first;
@@ -162,9 +163,9 @@ int cbm_plan_set_multipliers(cbm_plan* plan, const float* d_multipliers, void* s
  * in the staged kernel (0: its default; several streams share each warp).
  * Changing chunk_nnz or hot_rows re-lays out the plan (synchronous). */
 enum {
-  CBM_VARIANT_AUTO = 0,     /* staged where it applies, else register gather; register
-                               gather also for rows of at most 512 bytes when most rows
-                               hang below tree level 0 */
+  CBM_VARIANT_AUTO = 0,     /* staged for aligned rows of more than 32 16-byte vectors
+                               unless most rows hang below tree level 0, else register
+                               gather */
   CBM_VARIANT_REGISTER = 1, /* X rows gathered into registers, U entries at a time */
   CBM_VARIANT_STAGED = 2,   /* X rows staged through shared memory by cp.async */
   CBM_VARIANT_TMA = 3       /* X rows gathered four at a time by TMA (tile::gather4) into
