@@ -55,6 +55,7 @@ struct DirectArgs {
   float* y;        // [n_rows (n_cols for the transpose), c]
   int64_t c;
   float self_scale;
+  int32_t claim_runs;  // the SpMM's runs of rows are claimed (next_chunk, zeroed by direct_mark)
   int32_t self_term;  // y = fma(self_scale, x[i], (A x)[i]) in the SpMM store
   const int32_t* branches;
   int64_t n_branch_offsets;
@@ -74,7 +75,7 @@ __device__ __forceinline__ void record(QueueState* qs, int code, long long info)
 }
 
 __global__ void __launch_bounds__(kDirectThreads) direct_mark(const DirectArgs a) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) a.qs->next_row = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.qs->next_row = a.qs->next_chunk = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < a.n_edges; e += stride) {
     const int32_t u = a.src[e], v = a.dst[e];
@@ -92,94 +93,364 @@ __global__ void __launch_bounds__(kDirectThreads) direct_mark(const DirectArgs a
   }
 }
 
-// Team of TL lanes per row; lane owns VPL vectors of V floats per pass of
-// TL * VPL * V columns.
-template <int TL, int VPL, int V>
-__global__ void __launch_bounds__(kDirectThreads, 4) direct_spmm(const DirectArgs a) {
-  constexpr int kTeams = kDirectThreads / TL;
-  constexpr int U = (VPL * V >= 8) ? 4 : 8;  // entries whose gathers are in flight together
-  constexpr int64_t kPass = (int64_t)TL * VPL * V;
-  const int tl = threadIdx.x % TL;
-  const int64_t n_teams = (int64_t)gridDim.x * kTeams;
-  for (int64_t row = (int64_t)blockIdx.x * kTeams + threadIdx.x / TL; row < a.n_rows; row += n_teams) {
-    int64_t b = a.rp_b[row], e = a.rp_e[row];
-    if (b < 0 || e < b || e > a.nnz) {
-      if (tl == 0) record(a.qs, CBM_ERR_INDEX, row);
-      b = e = 0;
+// ---- direct_spmm ------------------------------------------------------------------
+// A row's sum is one chain of FMAs in entry order, so a long row cannot be
+// split by entries; it is split by columns instead, and its gathers run far
+// ahead of its FMAs.  A block takes a run of rows, lists the long ones, and its
+// warps draw tasks: first every (giant row, slice of 32 columns), then every
+// (long row, slice of 128), then the other rows, a team of TL lanes each.
+// Narrow slices put a giant's chain on more warps; wide ones cost a third of
+// the instructions per byte.
+//
+// Bound: the X-row gathers (L2, and DRAM where X is larger), with the longest
+// rows' chains behind them.  Fused-update products on B200, every row by one
+// team with four gathers in flight -> as here (us, bit-identical): 250,000-node
+// power-law graph of mean degree 20, 256 columns 1933 -> 840, a million nodes
+// 6330 -> 3380; 100,000 nodes of mean degree 14, 128 / 40 columns 692 / 546 ->
+// 311 / 229; 20,000 nodes, one column 146 -> 87.
+//
+// Long: more than 16 entries (256 columns: 840 us, 876 from 32 and 927 from
+// 64), 64 where a row fills no slice of 32 columns (4 columns: 123 us against
+// 152).  Giant: more than 512 entries, 256 up to 128 columns, which have one
+// wide slice only (7 columns: 175 us against 187).
+__device__ __forceinline__ int long_len(int64_t c) { return c >= 32 ? 16 : 64; }
+__device__ __forceinline__ int giant_len(int64_t c) { return c > 128 ? 512 : 256; }
+// Ring of a slice task: a giant's holds 6 groups of 8 entries x 128 bytes of X
+// rows and their weights (40 entries in flight while 8 are summed), a long
+// row's 3 groups of 4 entries x 512 bytes.
+constexpr int kRingGroups = 6;
+constexpr int kRingEntries = 8 * kRingGroups;
+constexpr int kRingFloats = kRingEntries * 33;  // 32 columns and a weight each
+constexpr int kWideGroups = 3;
+static_assert(kWideGroups * 4 * 128 <= kRingFloats, "one ring serves both");
+constexpr int kDirectWarps = kDirectThreads / 32;
+
+// One entry of a slice task: its column (-1 past the end, or out of range and
+// recorded) and its weight.
+__device__ __forceinline__ void slice_entry(const DirectArgs& a, int b, int n, int64_t c0, int k, int32_t& c,
+                                            float& w) {
+  c = -1;
+  w = 0.f;
+  if (k < n) {
+    c = __ldg(a.col + b + k);
+    w = a.val ? __ldg(a.val + b + k) : 1.f;
+    if (c < 0 || c >= a.n_cols) {
+      if (c0 == 0) record(a.qs, CBM_ERR_INDEX, b + k);
+      c = -1;
+      w = 0.f;
     }
-    for (int64_t c0 = 0; c0 < a.c; c0 += kPass) {
-      float acc[VPL][V];
+  }
+}
+
+template <int V>
+__device__ __forceinline__ void cp_async_piece(float* smem, const float* gmem, bool valid) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(smem);
+  if constexpr (V == 4) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gmem), "r"(valid ? 16u : 0u) : "memory");
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(gmem), "r"(valid ? 4u : 0u) : "memory");
+  }
+}
+
+// Giant rows: columns [c0, c0 + 32) of row `row`, entries [b, b + n), by one warp: X-row
+// pieces come through the warp's ring by cp.async, each lane then sums one
+// column.  An entry whose column is out of range (recorded) copies nothing and
+// weighs 0: its zero-filled slot leaves the sum as it is.
+template <int V>
+__device__ __forceinline__ void hub_slice(const DirectArgs& a, int64_t row, int b, int n, int64_t c0, float* ring) {
+  constexpr int kPieces = 32 / V;     // lanes that copy one entry's 32 columns
+  constexpr int kAtOnce = 32 / kPieces;  // entries per copy instruction
+  const int lane = threadIdx.x & 31;
+  const int piece = lane % kPieces, sub = lane / kPieces;
+  const bool in = c0 + piece * V < a.c;
+  float* weights = ring + kRingEntries * 32;
+  const float* x0 = a.x + c0 + (in ? piece * V : 0);
+  // entries come in batches of 32, one per lane, the next batch loaded ahead
+  int32_t col = 0, col_n = 0;
+  float w = 0.f, w_n = 0.f;
+  slice_entry(a, b, n, c0, lane, col, w);
+  slice_entry(a, b, n, c0, 32 + lane, col_n, w_n);
+  const int groups = (n + 7) / 8;
+  int made = 0;  // groups issued
+  auto produce = [&]() {
+    if (made < groups) {
+      if (made > 0 && (made & 3) == 0) {  // a new batch of 32 entries
+        col = col_n;
+        w = w_n;
+        slice_entry(a, b, n, c0, (made + 4) * 8 + lane, col_n, w_n);
+      }
+      const int slot = made % kRingGroups * 8, e0 = (made & 3) * 8;
+      const float we = __shfl_sync(0xffffffffu, w, e0 + (lane & 7));
+      if (lane < 8) weights[slot + lane] = we;
 #pragma unroll
-      for (int q = 0; q < VPL; ++q)
+      for (int u = 0; u < 8; u += kAtOnce) {
+        const int32_t c = __shfl_sync(0xffffffffu, col, e0 + u + sub);
+        cp_async_piece<V>(ring + (slot + u + sub) * 32 + piece * V, x0 + (int64_t)(c < 0 ? 0 : c) * a.c,
+                          in && c >= 0);
+      }
+    }
+    cp_async_commit();
+    ++made;
+  };
+#pragma unroll 1
+  for (int g = 0; g < kRingGroups - 1; ++g) produce();
+  float acc = 0.f;
+#pragma unroll 1
+  for (int g = 0; g < groups; ++g) {
+    produce();  // into the slot that the previous step summed
+    cp_async_wait<kRingGroups - 1>();
+    __syncwarp();
+    const float* slot = ring + g % kRingGroups * 8 * 32;
+    const float* ws = weights + g % kRingGroups * 8;
 #pragma unroll
-        for (int j = 0; j < V; ++j) acc[q][j] = 0.f;
-      // wide rows (groups of 4): the next group's columns and values are
-      // loaded while the current group's X rows are gathered; narrow rows
-      // (groups of 8) load each group's own at its start, which keeps their
-      // registers within four blocks per SM
-      constexpr bool kPrefetch = U == 4;
-      int32_t pc[U];
-      float pw[U];
-      auto fetch = [&](int64_t k) {
+    for (int u = 0; u < 8; ++u) acc = fmaf(ws[u], slot[u * 32 + lane], acc);
+    __syncwarp();
+  }
+  cp_async_wait<0>();
+  __syncwarp();
+  if (c0 + lane < a.c) {
+    const int64_t at = row * a.c + c0 + lane;
+    a.y[at] = a.self_term ? fmaf(a.self_scale, __ldg(a.x + at), acc) : acc;
+  }
+}
+
+// Long rows: columns [c0, c0 + 128), four per lane (one vector, or every 32nd
+// scalar).  A lane copies and sums only its own pieces, so its own cp.async
+// groups are all it waits for.
+template <int V>
+__device__ __forceinline__ void wide_slice(const DirectArgs& a, int64_t row, int b, int n, int64_t c0, float* ring) {
+  constexpr int P = 4 / V;  // pieces per lane
+  const int lane = threadIdx.x & 31;
+  int32_t col = 0, col_n = 0;
+  float w = 0.f, w_n = 0.f, w_p = 0.f;  // weights of the producer's batch of 32, the next and the previous one
+  slice_entry(a, b, n, c0, lane, col, w);
+  slice_entry(a, b, n, c0, 32 + lane, col_n, w_n);
+  const float* x0 = a.x + c0 + (c0 + lane * V < a.c ? lane * V : 0);
+  bool in[P];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-          const bool in = k + u < e;
-          pc[u] = in ? __ldg(a.col + k + u) : 0;
-          pw[u] = (in && a.val) ? __ldg(a.val + k + u) : 1.f;
-        }
-      };
-      if (kPrefetch && b < e) fetch(b);
-      for (int64_t k0 = b; k0 < e; k0 += U) {
-        const int n = (int)((e - k0) < U ? (e - k0) : U);
-        int64_t off[U];
-        float w[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          off[u] = -1;
-          w[u] = 0.f;
-          if (u < n) {
-            const int32_t cj = kPrefetch ? pc[u] : __ldg(a.col + k0 + u);
-            if (cj < 0 || cj >= a.n_cols) {
-              if (tl == 0) record(a.qs, CBM_ERR_INDEX, k0 + u);
-            } else {
-              off[u] = (int64_t)cj * a.c;
-              w[u] = kPrefetch ? pw[u] : (a.val ? __ldg(a.val + k0 + u) : 1.f);
-            }
-          }
-        }
-        if (kPrefetch && k0 + U < e) fetch(k0 + U);
-        float xv[U][VPL][V];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-          for (int q = 0; q < VPL; ++q) {
-            const int64_t cc = c0 + ((int64_t)q * TL + tl) * V;
-            if (off[u] >= 0 && cc < a.c) {
-              Vec<float, V>::load(a.x + off[u] + cc, xv[u][q]);
-            } else {
-#pragma unroll
-              for (int j = 0; j < V; ++j) xv[u][q][j] = 0.f;
-            }
-          }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (off[u] >= 0)
-#pragma unroll
-            for (int q = 0; q < VPL; ++q)
-#pragma unroll
-              for (int j = 0; j < V; ++j) acc[q][j] = fmaf(w[u], xv[u][q][j], acc[q][j]);
+  for (int q = 0; q < P; ++q) in[q] = c0 + (q * 32 + lane) * V < a.c;
+  const int groups = (n + 3) / 4;
+  int made = 0;  // groups issued
+  auto produce = [&](int slot) {
+    if (made < groups) {
+      if (made > 0 && (made & 7) == 0) {
+        w_p = w;
+        col = col_n;
+        w = w_n;
+        slice_entry(a, b, n, c0, (made + 8) * 4 + lane, col_n, w_n);
       }
 #pragma unroll
-      for (int q = 0; q < VPL; ++q) {
-        const int64_t cc = c0 + ((int64_t)q * TL + tl) * V;
-        if (cc >= a.c) continue;
-        if (a.self_term) {
-          float xs[V];
-          Vec<float, V>::load(a.x + row * a.c + cc, xs);
+      for (int u = 0; u < 4; ++u) {
+        const int32_t c = __shfl_sync(0xffffffffu, col, (made & 7) * 4 + u);
+        const float* xr = x0 + (int64_t)(c < 0 ? 0 : c) * a.c;
 #pragma unroll
-          for (int j = 0; j < V; ++j) acc[q][j] = fmaf(a.self_scale, xs[j], acc[q][j]);
+        for (int q = 0; q < P; ++q)
+          cp_async_piece<V>(ring + (slot * 4 + u) * 128 + (q * 32 + lane) * V, xr + (in[q] ? q * 32 : 0),
+                            in[q] && c >= 0);
+      }
+    }
+    cp_async_commit();
+    ++made;
+  };
+#pragma unroll
+  for (int g = 0; g < kWideGroups - 1; ++g) produce(g);
+  float acc[P][V];
+#pragma unroll
+  for (int q = 0; q < P; ++q)
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[q][j] = 0.f;
+  int slot = 0;
+#pragma unroll 1
+  for (int g = 0; g < groups; ++g) {
+    produce(slot == 0 ? kWideGroups - 1 : slot - 1);  // into the slot that the previous step summed
+    cp_async_wait<kWideGroups - 1>();
+    // the producer, at most 3 groups ahead, may be one batch of 8 groups on
+    const int last = (made < groups ? made : groups) - 1;
+    const float ws = last / 8 == g / 8 ? w : w_p;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float wu = __shfl_sync(0xffffffffu, ws, (g & 7) * 4 + u);
+#pragma unroll
+      for (int q = 0; q < P; ++q) {
+        const float* xs = ring + (slot * 4 + u) * 128 + (q * 32 + lane) * V;
+        if constexpr (V == 4) {
+          const float4 t = *reinterpret_cast<const float4*>(xs);
+          acc[q][0] = fmaf(wu, t.x, acc[q][0]);
+          acc[q][1] = fmaf(wu, t.y, acc[q][1]);
+          acc[q][2] = fmaf(wu, t.z, acc[q][2]);
+          acc[q][3] = fmaf(wu, t.w, acc[q][3]);
+        } else {
+          acc[q][0] = fmaf(wu, xs[0], acc[q][0]);
         }
-        store_vec<float, V>(a.y + row * a.c + cc, acc[q]);
+      }
+    }
+    slot = slot + 1 == kWideGroups ? 0 : slot + 1;
+  }
+  cp_async_wait<0>();
+#pragma unroll
+  for (int q = 0; q < P; ++q) {
+    if (!in[q]) continue;
+    const int64_t at = row * a.c + c0 + (q * 32 + lane) * V;
+    if (a.self_term) {
+      float xs[V];
+      Vec<float, V>::load(a.x + at, xs);
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[q][j] = fmaf(a.self_scale, xs[j], acc[q][j]);
+    }
+    store_vec<float, V>(a.y + at, acc[q]);
+  }
+}
+
+// One row by a team of TL lanes; a lane owns VPL vectors of V floats per pass
+// of TL * VPL * V columns.
+template <int TL, int VPL, int V>
+__device__ __forceinline__ void team_row(const DirectArgs& a, int64_t row, int64_t b, int64_t e, int tl) {
+  constexpr int U = (VPL * V >= 8) ? 4 : 8;  // entries whose gathers are in flight together
+  constexpr int64_t kPass = (int64_t)TL * VPL * V;
+  for (int64_t c0 = 0; c0 < a.c; c0 += kPass) {
+    float acc[VPL][V];
+#pragma unroll
+    for (int q = 0; q < VPL; ++q)
+#pragma unroll
+      for (int j = 0; j < V; ++j) acc[q][j] = 0.f;
+    // wide rows (groups of 4): the next group's columns and values are
+    // loaded while the current group's X rows are gathered; narrow rows
+    // (groups of 8) load each group's own at its start, which keeps their
+    // registers within four blocks per SM
+    constexpr bool kPrefetch = U == 4;
+    int32_t pc[U];
+    float pw[U];
+    auto fetch = [&](int64_t k) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const bool in = k + u < e;
+        pc[u] = in ? __ldg(a.col + k + u) : 0;
+        pw[u] = (in && a.val) ? __ldg(a.val + k + u) : 1.f;
+      }
+    };
+    if (kPrefetch && b < e) fetch(b);
+    for (int64_t k0 = b; k0 < e; k0 += U) {
+      const int n = (int)((e - k0) < U ? (e - k0) : U);
+      int64_t off[U];
+      float w[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        off[u] = -1;
+        w[u] = 0.f;
+        if (u < n) {
+          const int32_t cj = kPrefetch ? pc[u] : __ldg(a.col + k0 + u);
+          if (cj < 0 || cj >= a.n_cols) {
+            if (tl == 0) record(a.qs, CBM_ERR_INDEX, k0 + u);
+          } else {
+            off[u] = (int64_t)cj * a.c;
+            w[u] = kPrefetch ? pw[u] : (a.val ? __ldg(a.val + k0 + u) : 1.f);
+          }
+        }
+      }
+      if (kPrefetch && k0 + U < e) fetch(k0 + U);
+      float xv[U][VPL][V];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int q = 0; q < VPL; ++q) {
+          const int64_t cc = c0 + ((int64_t)q * TL + tl) * V;
+          if (off[u] >= 0 && cc < a.c) {
+            Vec<float, V>::load(a.x + off[u] + cc, xv[u][q]);
+          } else {
+#pragma unroll
+            for (int j = 0; j < V; ++j) xv[u][q][j] = 0.f;
+          }
+        }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (off[u] >= 0)
+#pragma unroll
+          for (int q = 0; q < VPL; ++q)
+#pragma unroll
+            for (int j = 0; j < V; ++j) acc[q][j] = fmaf(w[u], xv[u][q][j], acc[q][j]);
+    }
+#pragma unroll
+    for (int q = 0; q < VPL; ++q) {
+      const int64_t cc = c0 + ((int64_t)q * TL + tl) * V;
+      if (cc >= a.c) continue;
+      if (a.self_term) {
+        float xs[V];
+        Vec<float, V>::load(a.x + row * a.c + cc, xs);
+#pragma unroll
+        for (int j = 0; j < V; ++j) acc[q][j] = fmaf(a.self_scale, xs[j], acc[q][j]);
+      }
+      store_vec<float, V>(a.y + row * a.c + cc, acc[q]);
+    }
+  }
+}
+
+template <int TL, int VPL, int V>
+__global__ void __launch_bounds__(kDirectThreads, 4) direct_spmm(const DirectArgs a) {
+  extern __shared__ __align__(16) float rings[];
+  // a run's rows; giants listed from the front of s_long, long rows from its end
+  __shared__ int s_beg[kDirectThreads], s_len[kDirectThreads], s_long[kDirectThreads];
+  __shared__ int s_giants, s_longs, s_task;
+  __shared__ unsigned s_run;
+  constexpr int kTeams = kDirectThreads / TL;
+  constexpr int kPerWarp = 32 / TL;  // rows of one row task
+  // rows per run: one per team, up to four where every block then still gets
+  // several runs.  Runs are claimed in turn in the forms with a tree, whose
+  // calls own the workspace (direct_mark zeroed the counter); the others may
+  // share it with products on other streams and deal their runs out instead.
+  const int64_t per_team = a.n_rows / ((int64_t)gridDim.x * kTeams * 4);
+  const int run = kTeams * (int)(TL < 4 || per_team < 1 ? 1 : per_team < 4 ? per_team : 4);
+  const int lane = threadIdx.x & 31;
+  const int tl = lane % TL;
+  float* ring = rings + (threadIdx.x >> 5) * kRingFloats;
+  const int long_row = long_len(a.c), giant = giant_len(a.c);
+  const int narrow = (int)((a.c + 31) / 32), wide = (int)((a.c + 127) / 128);
+  for (unsigned turn = blockIdx.x;; turn += gridDim.x) {
+    __syncthreads();  // the previous run's lists are no longer read
+    if (threadIdx.x == 0) {
+      s_giants = s_longs = s_task = 0;
+      s_run = a.claim_runs ? atomicAdd(&a.qs->next_chunk, 1u) : turn;
+    }
+    __syncthreads();
+    const int64_t r0 = (int64_t)s_run * run;
+    if (r0 >= a.n_rows) break;
+    if ((int)threadIdx.x < run) {
+      const int64_t row = r0 + threadIdx.x;
+      int64_t b = 0, e = 0;
+      const bool have = row < a.n_rows;
+      if (have) {
+        b = a.rp_b[row], e = a.rp_e[row];
+        if (b < 0 || e < b || e > a.nnz) {
+          record(a.qs, CBM_ERR_INDEX, row);
+          b = e = 0;
+        }
+      }
+      s_beg[threadIdx.x] = (int)b;
+      s_len[threadIdx.x] = have ? (int)(e - b) : -1;
+      if (e - b > giant)
+        s_long[atomicAdd(&s_giants, 1)] = threadIdx.x;
+      else if (e - b > long_row)
+        s_long[kDirectThreads - 1 - atomicAdd(&s_longs, 1)] = threadIdx.x;
+    }
+    __syncthreads();
+    const int64_t giant_tasks = (int64_t)s_giants * narrow, long_tasks = giant_tasks + (int64_t)s_longs * wide;
+    const int64_t tasks = long_tasks + run / kPerWarp;
+    for (;;) {
+      int task = 0;
+      if (lane == 0) task = atomicAdd(&s_task, 1);
+      task = __shfl_sync(0xffffffffu, task, 0);
+      if (task >= tasks) break;
+      if (task < giant_tasks) {
+        const int i = s_long[task / narrow];
+        hub_slice<V>(a, r0 + i, s_beg[i], s_len[i], (int64_t)(task % narrow) * 32, ring);
+      } else if (task < long_tasks) {
+        const int k = task - (int)giant_tasks;
+        const int i = s_long[kDirectThreads - 1 - k / wide];
+        wide_slice<V>(a, r0 + i, s_beg[i], s_len[i], (int64_t)(k % wide) * 128, ring);
+      } else {
+        const int i = (task - (int)long_tasks) * kPerWarp + lane / TL;
+        if (s_len[i] >= 0 && s_len[i] <= long_row)
+          team_row<TL, VPL, V>(a, r0 + i, s_beg[i], (int64_t)s_beg[i] + s_len[i], tl);
+        __syncwarp();
       }
     }
   }
@@ -294,10 +565,10 @@ int current_device() {
 }
 
 template <typename K>
-int launch_direct(GridCache& cache, K kern, const DirectArgs& a, cudaStream_t st) {
-  const int grid = cached_grid(cache, kern, current_device(), kDirectThreads, 0);
+int launch_direct(GridCache& cache, K kern, const DirectArgs& a, cudaStream_t st, int smem = 0) {
+  const int grid = cached_grid(cache, kern, current_device(), kDirectThreads, smem);
   if (grid <= 0) return CBM_ERR_CUDA;
-  kern<<<grid, kDirectThreads, 0, st>>>(a);
+  kern<<<grid, kDirectThreads, smem, st>>>(a);
   return cuda_status(cudaGetLastError());
 }
 
@@ -307,7 +578,8 @@ template <int TL, int VPL, int V>
 int launch_shape(int which, const DirectArgs& a, cudaStream_t st) {
   static GridCache c_spmm, c_update, c_spmm_t;
   switch (which) {
-    case K_SPMM: return launch_direct(c_spmm, direct_spmm<TL, VPL, V>, a, st);
+    case K_SPMM:
+      return launch_direct(c_spmm, direct_spmm<TL, VPL, V>, a, st, kDirectWarps * kRingFloats * (int)sizeof(float));
     case K_UPDATE: return launch_direct(c_update, direct_update<TL, VPL, V>, a, st);
     default: return launch_direct(c_spmm_t, direct_spmm_t<TL, VPL, V>, a, st);
   }
@@ -417,6 +689,7 @@ int run(const DirectCall& k) {
     direct_mark<<<sm_count(current_device()) * 4, kDirectThreads, 0, st>>>(a);
     if ((rc = cuda_status(cudaGetLastError()))) return rc;
     a.n_rows = k.spmm ? k.n_rows : k.n_y_rows;
+    a.claim_runs = 1;
   }
   if (k.spmm && k.transpose) {
     if (cudaMemsetAsync(k.y, 0, (size_t)(k.n_y_rows * k.c * 4), st) != cudaSuccess) return CBM_ERR_CUDA;
