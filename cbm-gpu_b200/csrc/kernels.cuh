@@ -27,7 +27,6 @@
 namespace cbm {
 
 constexpr int kThreads = 256;
-
 // Forward entry word: column in bits 0-29, bit 30 set for the columns gathered
 // most often (L2 keeps their X rows), bit 31 the sign.
 constexpr uint32_t kColMask = 0x3fffffffu;
@@ -197,6 +196,16 @@ struct Vec<__nv_bfloat16, 8> {
   }
 };
 template <>
+struct Vec<__nv_bfloat16, 4> {
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[4]) {
+    const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
+    o[0] = __uint_as_float(t.x << 16);
+    o[1] = __uint_as_float(t.x & 0xffff0000u);
+    o[2] = __uint_as_float(t.y << 16);
+    o[3] = __uint_as_float(t.y & 0xffff0000u);
+  }
+};
+template <>
 struct Vec<__nv_bfloat16, 1> {
   static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[1]) {
     const unsigned short b = __ldg(reinterpret_cast<const unsigned short*>(p));
@@ -227,6 +236,11 @@ __device__ __forceinline__ void store_vec<__nv_bfloat16, 8>(__nv_bfloat16* p, co
 #pragma unroll
   for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
   *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
+}
+template <>
+__device__ __forceinline__ void store_vec<__nv_bfloat16, 4>(__nv_bfloat16* p, const float (&v)[4]) {
+  __nv_bfloat162 h[2] = {__floats2bfloat162_rn(v[0], v[1]), __floats2bfloat162_rn(v[2], v[3])};
+  *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(h);
 }
 template <>
 __device__ __forceinline__ void store_vec<__nv_bfloat16, 1>(__nv_bfloat16* p, const float (&v)[1]) {
@@ -389,6 +403,14 @@ struct Lane {
   }
 };
 
+// Lanes per team as a template parameter (TLC): 32, or one of these.
+constexpr int kTeamAny = 0;   // run-time team size; entries come by shuffles
+// run-time team size of one or two lanes: a batch of one entry per lane would
+// be less than a group, so every lane reads its team's entries itself (100,000
+// nodes, one FP32 column: 268 -> 172 us, 8 BF16 columns 231 -> 160; with four
+// lanes shuffles are faster, 16 FP32 columns 96 against 119)
+constexpr int kTeamNarrow = 1;
+
 // acc += sum of scale_k * X[col_k] over the `len` entries of ent, in order, one
 // FMA each.  Every lane of the warp calls it: the trip counts come from wlen,
 // the largest len of the warp's teams, so teams that share a warp step through
@@ -405,11 +427,59 @@ __device__ __forceinline__ void gather_row(float (&acc)[VPL][V], const Lane<XT, 
                                            const float* __restrict__ mult, int tl, int team_lanes, Between between) {
   constexpr int U = reg_in_flight<XT, VPL, V>();
   using R = Raw<XT, V>;
-  const int TL = TLC ? TLC : team_lanes;
+  const int TL = TLC == 32 ? 32 : team_lanes;
   if (wlen <= 0) {
     between();
     return;
   }
+  if constexpr (TLC == kTeamNarrow) {
+    // one address per team; the next group's entries load a group ahead
+    uint32_t eg[U];
+    float sg[U];
+    auto fetch = [&](int j) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        eg[u] = 0;
+        sg[u] = 0.f;
+        if (j + u < len) {
+          eg[u] = __ldg(ent + j + u);
+          if (vals) sg[u] = __ldg(vals + j + u);
+        }
+      }
+    };
+    fetch(0);
+#pragma unroll 1
+    for (int j = 0; j < wlen; j += U) {
+      typename R::type raw[U][VPL];
+      float sc[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const char* row = ln.row(eg[u] & kColMask);
+        if (j + u < len) {
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) raw[u][v] = R::load(reinterpret_cast<const XT*>(row + ln.off[v]));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        sc[u] = vals ? sg[u] : j + u < len ? reg_scale(eg[u], nullptr, 0, scale_mode, mult) : 0.f;
+      if (j == 0) between();
+      if (j + U < wlen) fetch(j + U);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (j + u < len) {
+          const float su = __fmul_rn(sc[u], dv);
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) {
+            float t[V];
+            R::widen(raw[u][v], t);
+#pragma unroll
+            for (int k = 0; k < V; ++k) acc[v][k] = fmaf(su, t[k], acc[v][k]);
+          }
+        }
+      }
+    }
+  } else {
   for (int b = 0; b < wlen; b += TL) {
     const int in = b + TL + tl;
     uint32_t en = 0;
@@ -474,6 +544,7 @@ __device__ __forceinline__ void gather_row(float (&acc)[VPL][V], const Lane<XT, 
     e = en;
     if (!vals) sn = in < len ? reg_scale(en, vals, in, scale_mode, mult) : 0.f;
     s = __fmul_rn(sn, dv);
+  }
   }
 }
 
@@ -568,7 +639,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
   // parents' rows come from the FP32 state rows
   const bool state = sizeof(YT) != 4 || FORM == FORM_GIN || (COMP && a.gin);
   const int lane = threadIdx.x & 31;
-  const int TL = TLC ? TLC : a.team;
+  const int TL = TLC == 32 ? 32 : a.team;
   const int tl = lane & (TL - 1);
   const int team = lane / TL;
   const unsigned teams = 32 / TL;
@@ -1735,16 +1806,14 @@ struct RevArgs {
   // items, deepest level first: for each internal node its chunk items (long
   // children lists), then the node item
   int32_t n_items;
-  const int32_t* node;   // node id, or -1 for a chunk item
-  const int32_t* slot;   // node item: internal slot; chunk item: chunk id
-  const int64_t* ptr;    // children (or chunk) ranges in ent
+  const int4* meta;      // x = node, -1 for a chunk item; y = internal slot or chunk id;
+                         // z = first child and w = children, or first chunk and minus the chunks
   const uint32_t* ent;   // child | internal bit (slot then)
-  const int32_t* chunk0; // node item: first chunk id, -1 when not split
-  const int32_t* nchunk; // node item: number of chunks
   const float* mult;
   int32_t scale_g;       // G' = m o G
   unsigned int* flag;    // [n_internal]
   unsigned int* chunk_flag;  // [chunks]
+  unsigned int* claims;  // kClaimQueues counters
   float* partial;        // [chunks, ldp]
   QueueState* qs;
   const void* g;
@@ -1753,20 +1822,19 @@ struct RevArgs {
   int32_t ldp;
   int32_t nvec;
   int32_t team;
-  int32_t rows_per_claim;
   long long timeout_ns;
 };
 
 struct TrArgs {
   int32_t n_items;       // columns of Delta
-  const int64_t* ptr;
+  const int4* meta;      // per item, longest lists first: x = column, z = first
+                         // entry and w = entries, or first chunk and minus the chunks
   const uint32_t* ent;   // row | internal bit (slot then) | sign << 31
   int32_t n_chunks;
-  const int32_t* chunk0;
-  const int32_t* chunk_item;
   const int64_t* chunk_beg;
   const int64_t* chunk_end;
   unsigned int* chunk_flag;
+  unsigned int* claims;  // kClaimQueues counters
   const float* mult;
   int32_t scale_g;       // leaves read m[v] * G[v]
   int32_t scale_out;     // dX[j] *= m[j]
@@ -1780,39 +1848,34 @@ struct TrArgs {
   int32_t nvec;
   float* partial;
   int32_t team;
-  int32_t rows_per_claim;
   long long timeout_ns;
 };
 
-// acc += sum over entries of s * (internal ? H[slot] : scale * G[row]).  With
-// wait != 0 each internal entry's ready flag is awaited first.
+// acc += sum over the `len` children in ent of (internal ? H[slot] : scale * G[row]),
+// each internal child's ready flag awaited first.  e: the lane's child of the
+// first TL; later batches of TL load one batch ahead.
 template <typename GT, int VPL, int V>
-__device__ __forceinline__ void gather_dual(float (&acc)[VPL][V], const GT* __restrict__ g, int64_t ldg,
-                                            const float* __restrict__ h, int ldp, int nvec,
-                                            const uint32_t* __restrict__ ent, int64_t beg, int64_t end,
-                                            const float* __restrict__ mult, bool scale_g, bool signed_ent,
-                                            const unsigned int* flag, unsigned epoch, QueueState* qs,
-                                            long long timeout_ns, int tl, int TL, unsigned tmask) {
+__device__ __forceinline__ void gather_children(float (&acc)[VPL][V], const RevArgs& a, const GT* __restrict__ g,
+                                                const uint32_t* __restrict__ ent, int len, uint32_t e, unsigned epoch,
+                                                int tl, int TL, unsigned tmask) {
   constexpr int U = unroll_for<VPL, V>();
-  for (int64_t base = beg; base < end; base += TL) {
-    const int64_t idx = base + tl;
-    uint32_t e = 0;
+  for (int base = 0; base < len; base += TL) {
+    const int at = base + TL + tl;
+    const uint32_t en = at < len ? __ldg(ent + at) : 0u;
+    const int cnt = len - base < TL ? len - base : TL;
     float sc = 0.f;
-    if (idx < end) {
-      e = __ldg(ent + idx);
+    if (tl < cnt) {
       const uint32_t r = e & kIndexMask;
-      const float sgn = (signed_ent && (e >> 31)) ? -1.f : 1.f;
       if (e & kInternalBit) {
-        sc = sgn;
+        sc = 1.f;
         // each lane acquires the flag of its own entry; the team barrier below
         // orders every lane's later reads of those rows after these acquires
-        if (flag) wait_flag(flag + r, epoch, qs, timeout_ns, (long long)r);
+        wait_flag(a.flag + r, epoch, a.qs, a.timeout_ns, (long long)r);
       } else {
-        sc = scale_g ? sgn * __ldg(mult + r) : sgn;
+        sc = a.scale_g ? __ldg(a.mult + r) : 1.f;
       }
     }
-    if (flag) __syncwarp(tmask);
-    const int cnt = (int)((end - base) < TL ? (end - base) : TL);
+    __syncwarp(tmask);
     for (int j = 0; j < cnt; j += U) {
       float buf[U][VPL][V];
       float s[U];
@@ -1826,11 +1889,11 @@ __device__ __forceinline__ void gather_dual(float (&acc)[VPL][V], const GT* __re
 #pragma unroll
         for (int v = 0; v < VPL; ++v) {
           const int vi = tl + v * TL;
-          if (j + u < cnt && vi < nvec) {
+          if (j + u < cnt && vi < a.nvec) {
             if (in) {
-              load_f32_cg<V>(h + row_off(r, ldp) + vi * V, buf[u][v]);
+              load_f32_cg<V>(a.h + row_off(r, a.ldp) + vi * V, buf[u][v]);
             } else {
-              Vec<GT, V>::load(g + row_off(r, ldg) + (int64_t)vi * V, buf[u][v]);
+              Vec<GT, V>::load(g + row_off(r, a.ldg) + (int64_t)vi * V, buf[u][v]);
             }
           } else {
 #pragma unroll
@@ -1848,103 +1911,41 @@ __device__ __forceinline__ void gather_dual(float (&acc)[VPL][V], const GT* __re
         }
       }
     }
-  }
-}
-
-// acc += sum over entries of s * (internal ? H[slot] : scale * G[row]) with the
-// whole warp on one entry range: G = 32 / TL groups of TL lanes, group g takes
-// the entries g, g + G, g + 2G, ... of each batch of 32, and the groups' sums
-// are added at the end (shuffles across the group bits), so every lane holds
-// the total.  Rows narrower than a warp then keep all 32 lanes on one column
-// instead of splitting the warp between columns whose lists differ in length.
-// The sum's order differs from the one-team order; the adjoint is held to
-// FP64 and finite-difference bounds, not to the forward's order.
-template <typename GT, int VPL, int V>
-__device__ __forceinline__ void gather_dual_split(float (&acc)[VPL][V], const GT* __restrict__ g, int64_t ldg,
-                                                  const float* __restrict__ h, int ldp, int nvec,
-                                                  const uint32_t* __restrict__ ent, int64_t beg, int64_t end,
-                                                  const float* __restrict__ mult, bool scale_g, int lane, int TL) {
-  constexpr int U = unroll_for<VPL, V>();
-  const int grp = lane / TL;
-  const int tl = lane & (TL - 1);
-  const int G = 32 / TL;
-  for (int64_t base = beg; base < end; base += 32) {
-    const int64_t idx = base + lane;
-    uint32_t e = 0;
-    float sc = 0.f;
-    if (idx < end) {
-      e = __ldg(ent + idx);
-      const uint32_t r = e & kIndexMask;
-      const float sgn = (e >> 31) ? -1.f : 1.f;
-      sc = (e & kInternalBit) ? sgn : (scale_g ? sgn * __ldg(mult + r) : sgn);
-    }
-    const int cnt = (int)((end - base) < 32 ? (end - base) : 32);
-    for (int j = 0; j < cnt; j += G * U) {  // the same trip count on every lane
-      float buf[U][VPL][V];
-      float s[U];
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const int jj = j + u * G + grp;
-        const uint32_t eu = __shfl_sync(0xffffffffu, e, jj < cnt ? jj : 0);
-        s[u] = __shfl_sync(0xffffffffu, sc, jj < cnt ? jj : 0);
-        const uint32_t r = eu & kIndexMask;
-        const bool in = (eu & kInternalBit) != 0;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const int vi = tl + v * TL;
-          if (jj < cnt && vi < nvec) {
-            if (in) {
-              load_f32_cg<V>(h + row_off(r, ldp) + vi * V, buf[u][v]);
-            } else {
-              Vec<GT, V>::load(g + row_off(r, ldg) + (int64_t)vi * V, buf[u][v]);
-            }
-          } else {
-#pragma unroll
-            for (int k = 0; k < V; ++k) buf[u][v][k] = 0.f;
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        if (j + u * G + grp < cnt) {
-#pragma unroll
-          for (int v = 0; v < VPL; ++v)
-#pragma unroll
-            for (int k = 0; k < V; ++k) acc[v][k] = fmaf(s[u], buf[u][v][k], acc[v][k]);
-        }
-      }
-    }
-  }
-  for (int off = TL; off < 32; off <<= 1) {
-#pragma unroll
-    for (int v = 0; v < VPL; ++v)
-#pragma unroll
-      for (int k = 0; k < V; ++k) acc[v][k] += __shfl_xor_sync(0xffffffffu, acc[v][k], off);
+    e = en;
   }
 }
 
 template <typename GT, int VPL, int V>
 __global__ void __launch_bounds__(kThreads) rev_kernel(const RevArgs a) {
+  constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int TL = a.team;
   const int team = lane / TL;
   const int tl = lane & (TL - 1);
-  const int teams = 32 / TL;
-  const unsigned tmask = (TL == 32) ? 0xffffffffu : (((1u << TL) - 1u) << (team * TL));
+  const unsigned teams = 32 / TL;
+  const unsigned tmask = (TL == 32) ? kAll : (((1u << TL) - 1u) << (team * TL));
   const unsigned epoch = *(volatile unsigned*)&a.qs->epoch + 1u;
   const GT* g = static_cast<const GT*>(a.g);
-  const unsigned per_claim = (unsigned)(teams * a.rows_per_claim);
+  const unsigned n = (unsigned)a.n_items;
+  const unsigned wq = threadIdx.x >> 5;
   for (;;) {
-    unsigned base = 0;
-    if (lane == 0) base = atomicAdd(&a.qs->next_row, per_claim);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= (unsigned)a.n_items) break;
-    for (int rr = 0; rr < a.rows_per_claim; ++rr) {
-      const unsigned item = base + team + (unsigned)(rr * teams);
-      if (item >= (unsigned)a.n_items) break;
-      const int w = a.node[item];
-      const int ws = a.slot[item];
+    // one item per team and claim, and nothing claimed ahead: an item waits on
+    // children claimed just before it, and one held back behind another item of
+    // its warp holds up its parents (with a claim and a record made ahead, as in
+    // the forward kernel, 80 -> 94-112 us on the GCN graph)
+    unsigned g0 = 0;
+    if (lane == 0) g0 = atomicAdd(a.claims + wq * kClaimStride, 1u);
+    g0 = (__shfl_sync(kAll, g0, 0) * kClaimQueues + wq) * teams;
+    if (g0 >= n) break;
+    const int4 m0 = __ldg(a.meta + g0 + team);
+    const uint32_t e0 = tl < m0.w ? __ldg(a.ent + (uint32_t)m0.z + tl) : 0u;
+    if (g0 + team < n) {
+      const int w = m0.x;
       float acc[VPL][V];
+#pragma unroll
+      for (int v = 0; v < VPL; ++v)
+#pragma unroll
+        for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
       if (w >= 0) {
         // node item: its own G' row
         const float sw = a.scale_g ? __ldg(a.mult + w) : 1.f;
@@ -1953,17 +1954,13 @@ __global__ void __launch_bounds__(kThreads) rev_kernel(const RevArgs a) {
           const int vi = tl + v * TL;
           if (vi < a.nvec) {
             float t[V];
-            Vec<GT, V>::load(g + (int64_t)w * a.ldg + (int64_t)vi * V, t);
+            Vec<GT, V>::load(g + row_off(w, a.ldg) + (int64_t)vi * V, t);
 #pragma unroll
             for (int q = 0; q < V; ++q) acc[v][q] = __fmul_rn(sw, t[q]);
-          } else {
-#pragma unroll
-            for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
           }
         }
         // partial sums of its chunks, in order
-        const int c0 = a.chunk0[item];
-        for (int k = c0, ke = c0 + (c0 >= 0 ? a.nchunk[item] : 0); k < ke; ++k) {
+        for (int k = m0.z, ke = m0.z - m0.w; k < ke && m0.w < 0; ++k) {
           if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
           const float* prow = a.partial + (int64_t)k * a.ldp;
 #pragma unroll
@@ -1977,101 +1974,291 @@ __global__ void __launch_bounds__(kThreads) rev_kernel(const RevArgs a) {
             }
           }
         }
-      } else {
-#pragma unroll
-        for (int v = 0; v < VPL; ++v)
-#pragma unroll
-          for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
       }
-      gather_dual<GT, VPL, V>(acc, g, a.ldg, a.h, a.ldp, a.nvec, a.ent, a.ptr[item], a.ptr[item + 1], a.mult,
-                              a.scale_g != 0, false, a.flag, epoch, a.qs, a.timeout_ns, tl, TL, tmask);
-      float* orow = (w >= 0) ? a.h + (int64_t)ws * a.ldp : a.partial + (int64_t)ws * a.ldp;
+      gather_children<GT, VPL, V>(acc, a, g, a.ent + (uint32_t)m0.z, m0.w, e0, epoch, tl, TL, tmask);
+      float* orow = (w >= 0 ? a.h : a.partial) + (int64_t)m0.y * a.ldp;
 #pragma unroll
       for (int v = 0; v < VPL; ++v) {
         const int vi = tl + v * TL;
         if (vi < a.nvec) store_f32<V>(orow + vi * V, acc[v]);
       }
-      __threadfence();
+      // the barrier orders the team's stores before its first lane's release,
+      // which carries them (cumulativity)
       __syncwarp(tmask);
-      if (tl == 0) st_release((w >= 0 ? a.flag : a.chunk_flag) + ws, epoch);
+      if (tl == 0) st_release((w >= 0 ? a.flag : a.chunk_flag) + m0.y, epoch);
     }
     __syncwarp();
   }
-  finish_block(a.qs, epoch);
+  finish_block(a.qs, epoch, true, a.claims);
 }
 
-// SPLIT (rows narrower than a warp): one item per warp, its entries spread
-// over the warp's lane groups (gather_dual_split); group 0 writes the result.
-template <typename GT, typename DT, int VPL, int V, bool SPLIT = false>
-__global__ void __launch_bounds__(kThreads) tr_kernel(const TrArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int TL = a.team;
-  const int team = SPLIT ? 0 : lane / TL;
-  const int tl = lane & (TL - 1);
-  const int teams = SPLIT ? 1 : 32 / TL;
-  const bool writer = !SPLIT || lane < TL;
-  const unsigned tmask = (SPLIT || TL == 32) ? 0xffffffffu : (((1u << TL) - 1u) << (team * TL));
-  const unsigned epoch = *(volatile unsigned*)&a.qs->epoch + 1u;
-  const GT* g = static_cast<const GT*>(a.g);
-  if (a.n_chunks > 0) {
-    for (;;) {
-      unsigned base = 0;
-      if (lane == 0) base = atomicAdd(&a.qs->next_chunk, (unsigned)teams);
-      base = __shfl_sync(0xffffffffu, base, 0);
-      if (base >= (unsigned)a.n_chunks) break;
-      const unsigned k = base + team;
-      if (k < (unsigned)a.n_chunks) {
-        float acc[VPL][V];
-#pragma unroll
-        for (int v = 0; v < VPL; ++v)
-#pragma unroll
-          for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-        if constexpr (SPLIT) {
-          gather_dual_split<GT, VPL, V>(acc, g, a.ldg, a.h, a.ldp, a.nvec, a.ent, a.chunk_beg[k], a.chunk_end[k],
-                                        a.mult, a.scale_g != 0, lane, TL);
-        } else {
-          gather_dual<GT, VPL, V>(acc, g, a.ldg, a.h, a.ldp, a.nvec, a.ent, a.chunk_beg[k], a.chunk_end[k],
-                                  a.mult, a.scale_g != 0, true, nullptr, epoch, a.qs, a.timeout_ns, tl, TL,
-                                  tmask);
-        }
-        float* prow = a.partial + (int64_t)k * a.ldp;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const int vi = tl + v * TL;
-          if (writer && vi < a.nvec) store_f32<V>(prow + vi * V, acc[v]);
-        }
-        __threadfence();
-        __syncwarp(tmask);
-        if (SPLIT ? lane == 0 : tl == 0) st_release(a.chunk_flag + k, epoch);
-      }
-      __syncwarp();
-    }
+// V elements of a row of G (type GT) or of H (FP32) as loaded.  BF16 rows come in
+// vectors of four elements here, as H's do, so that a vector of either takes the
+// same registers (170,000 nodes, 128 columns: 361 us with vectors of eight,
+// 279 with four).
+template <typename GT, int V>
+struct Dual;
+template <int V>
+struct Dual<float, V> {
+  using type = typename Raw<float, V>::type;
+  static constexpr int regs = Raw<float, V>::regs;
+  static __device__ __forceinline__ type load(const char* g, const char* h, bool in) {
+    return Raw<float, V>::load(reinterpret_cast<const float*>(in ? h : g));
   }
-  const unsigned per_claim = (unsigned)(teams * a.rows_per_claim);
-  for (;;) {
-    unsigned base = 0;
-    if (lane == 0) base = atomicAdd(&a.qs->next_row, per_claim);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= (unsigned)a.n_items) break;
-    for (int rr = 0; rr < a.rows_per_claim; ++rr) {
-      const unsigned item = base + team + (unsigned)(rr * teams);
-      if (item >= (unsigned)a.n_items) break;
+  static __device__ __forceinline__ void widen(const type& r, bool, float (&o)[V]) { Raw<float, V>::widen(r, o); }
+};
+template <>
+struct Dual<__nv_bfloat16, 4> {
+  using type = uint4;
+  static constexpr int regs = 4;
+  static __device__ __forceinline__ type load(const char* g, const char* h, bool in) {
+    if (in) return __ldg(reinterpret_cast<const uint4*>(h));
+    const uint2 t = __ldg(reinterpret_cast<const uint2*>(g));
+    return make_uint4(t.x, t.y, 0u, 0u);
+  }
+  static __device__ __forceinline__ void widen(const type& r, bool in, float (&o)[4]) {
+    o[0] = __uint_as_float(in ? r.x : r.x << 16);
+    o[1] = __uint_as_float(in ? r.y : r.x & 0xffff0000u);
+    o[2] = __uint_as_float(in ? r.z : r.y << 16);
+    o[3] = __uint_as_float(in ? r.w : r.y & 0xffff0000u);
+  }
+};
+template <>
+struct Dual<__nv_bfloat16, 1> {
+  using type = uint32_t;
+  static constexpr int regs = 1;
+  static __device__ __forceinline__ type load(const char* g, const char* h, bool in) {
+    return in ? __ldg(reinterpret_cast<const uint32_t*>(h))
+              : (uint32_t)__ldg(reinterpret_cast<const unsigned short*>(g)) << 16;
+  }
+  static __device__ __forceinline__ void widen(const type& r, bool, float (&o)[1]) { o[0] = __uint_as_float(r); }
+};
+
+// Gathers in flight per lane: 16 registers' worth, at most 8 (170,000-node GCN
+// graph, 40 FP32 columns, the whole adjoint: 160 us, 177 with 32 registers).
+template <typename GT, int VPL, int V>
+__host__ __device__ constexpr int dual_in_flight() {
+  const int u = 16 / (VPL * Dual<GT, V>::regs);
+  return u < 1 ? 1 : (u > 8 ? 8 : u);
+}
+
+// Scale of one transposed entry: the sign, times m[row] for a leaf of a scaled G.
+__device__ __forceinline__ float dual_scale(uint32_t e, bool scale_g, const float* __restrict__ mult) {
+  const float sgn = (e >> 31) ? -1.f : 1.f;
+  return (!scale_g || (e & kInternalBit)) ? sgn : sgn * __ldg(mult + (e & kIndexMask));
+}
+
+// acc += sum of s * (internal ? H[slot] : G[row]) over `len` entries, in order:
+// gather_row (above) with a row source per entry.
+template <typename GT, int VPL, int V, int TLC, typename Between>
+__device__ __forceinline__ void gather_dual_row(float (&acc)[VPL][V], const Lane<GT, VPL, V, true>& lg,
+                                                const Lane<float, VPL, V, false>& lh,
+                                                const uint32_t* __restrict__ ent, int len, int wlen, uint32_t e,
+                                                float s, bool scale_g, const float* __restrict__ mult, int tl,
+                                                int team_lanes, Between between) {
+  constexpr int U = dual_in_flight<GT, VPL, V>();
+  using D = Dual<GT, V>;
+  const int TL = TLC == 32 ? 32 : team_lanes;
+  if (wlen <= 0) {
+    between();
+    return;
+  }
+  if constexpr (TLC == kTeamNarrow) {
+    uint32_t eg[U];
+    auto fetch = [&](int j) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) eg[u] = j + u < len ? __ldg(ent + j + u) : 0u;
+    };
+    fetch(0);
+#pragma unroll 1
+    for (int j = 0; j < wlen; j += U) {
+      typename D::type raw[U][VPL];
+      float sc[U];
+      bool in[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t r = eg[u] & kIndexMask;
+        in[u] = (eg[u] & kInternalBit) != 0;
+        if (j + u < len) {
+          const char* g = lg.row(r);
+          const char* h = lh.row(r);
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) raw[u][v] = D::load(g + lg.off[v], h + lh.off[v], in[u]);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) sc[u] = j + u < len ? dual_scale(eg[u], scale_g, mult) : 0.f;
+      if (j == 0) between();
+      if (j + U < wlen) fetch(j + U);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (j + u < len) {
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) {
+            float t[V];
+            D::widen(raw[u][v], in[u], t);
+#pragma unroll
+            for (int k = 0; k < V; ++k) acc[v][k] = fmaf(sc[u], t[k], acc[v][k]);
+          }
+        }
+      }
+    }
+  } else {
+  for (int b = 0; b < wlen; b += TL) {
+    const int at = b + TL + tl;
+    const uint32_t en = at < len ? __ldg(ent + at) : 0u;
+    const int cnt = len - b < TL ? len - b : TL;
+    const int wc = wlen - b < TL ? wlen - b : TL;
+#pragma unroll 1
+    for (int j = 0; j < wc; j += U) {
+      typename D::type raw[U][VPL];
+      uint32_t eu[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        eu[u] = __shfl_sync(0xffffffffu, e, j + u, TL);
+        const uint32_t r = eu[u] & kIndexMask;
+        const bool in = (eu[u] & kInternalBit) != 0;
+        if (j + u < cnt) {
+          const char* g = lg.row(r);
+          const char* h = lh.row(r);
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) raw[u][v] = D::load(g + lg.off[v], h + lh.off[v], in);
+        }
+      }
+      if (b + j == 0) between();
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const float su = __shfl_sync(0xffffffffu, s, j + u, TL);
+        if (j + u < cnt) {
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) {
+            float t[V];
+            D::widen(raw[u][v], (eu[u] & kInternalBit) != 0, t);
+#pragma unroll
+            for (int k = 0; k < V; ++k) acc[v][k] = fmaf(su, t[k], acc[v][k]);
+          }
+        }
+      }
+    }
+    e = en;
+    s = at < len ? dual_scale(en, scale_g, mult) : 0.f;
+  }
+  }
+}
+
+// (Measured, the whole adjoint on B200, a column per team or warp with every
+// load in turn -> as here: 170,000-node GCN graph, 40 FP32 columns 224 -> 160
+// us, 128 FP32 302 -> 203, 128 BF16 355 -> 279; 200,000 nodes on a shallow tree,
+// 64 / 256 columns 226 / 545 -> 163 / 416.)
+//
+// The transposed gather, a pipeline like the register forward kernel's: lists
+// of like length share a warp (the items are in length order), the next list's
+// record, entries and claim load under the current one's gathers, and the rows
+// are handed out from eight counters.  Where more than four teams share a warp,
+// it still takes four lists: each is split over its share of the teams, in
+// equal runs whose sums are added by shuffles (no order is kept here, the
+// adjoint is held to FP64), as is every chunk over all of them; the narrowest
+// teams would else walk their longest lists alone.
+template <typename GT, typename DT, int VPL, int V, int TLC>
+__global__ void __launch_bounds__(kThreads, (VPL > 2 ? 1 : VPL == 2 ? 2 : 3)) tr_kernel(const TrArgs a) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int TL = TLC == 32 ? 32 : a.team;
+  const int tl = lane & (TL - 1);
+  const int team = lane / TL;
+  const unsigned teams = 32 / TL;
+  const unsigned epoch = *(volatile unsigned*)&a.qs->epoch + 1u;
+  const Lane<GT, VPL, V, true> lg(a.g, a.ldg, a.nvec, tl, TL);
+  const Lane<float, VPL, V, false> lh(a.h, a.ldp, a.nvec, tl, TL);
+  const bool scale_g = a.scale_g != 0;
+  const unsigned n = (unsigned)a.n_items;
+  if (a.n_chunks > 0) {
+    unsigned pend = 0;
+    if (lane == 0) pend = atomicAdd(&a.qs->next_chunk, 1u);
+    for (;;) {
+      const unsigned k = __shfl_sync(kAll, pend, 0);
+      if (k >= (unsigned)a.n_chunks) break;
+      if (lane == 0) pend = atomicAdd(&a.qs->next_chunk, 1u);
+      const int all = (int)(a.chunk_end[k] - a.chunk_beg[k]);
+      const int run = (all + (int)teams - 1) >> (__ffs((int)teams) - 1);
+      const int from = team * run < all ? team * run : all;
+      const int len = all - from < run ? all - from : run;
+      const uint32_t* ent = a.ent + a.chunk_beg[k] + from;
+      const uint32_t e = tl < len ? __ldg(ent + tl) : 0u;
+      const float s = tl < len ? dual_scale(e, scale_g, a.mult) : 0.f;
       float acc[VPL][V];
 #pragma unroll
       for (int v = 0; v < VPL; ++v)
 #pragma unroll
         for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-      const int c0 = a.chunk0[item];
-      if (c0 < 0) {
-        if constexpr (SPLIT) {
-          gather_dual_split<GT, VPL, V>(acc, g, a.ldg, a.h, a.ldp, a.nvec, a.ent, a.ptr[item], a.ptr[item + 1],
-                                        a.mult, a.scale_g != 0, lane, TL);
-        } else {
-          gather_dual<GT, VPL, V>(acc, g, a.ldg, a.h, a.ldp, a.nvec, a.ent, a.ptr[item], a.ptr[item + 1], a.mult,
-                                  a.scale_g != 0, true, nullptr, epoch, a.qs, a.timeout_ns, tl, TL, tmask);
+      gather_dual_row<GT, VPL, V, TLC>(acc, lg, lh, ent, len, run, e, s, scale_g, a.mult, tl, TL, [] {});
+      for (int off = TL; off < 32; off <<= 1) {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+#pragma unroll
+          for (int q = 0; q < V; ++q) acc[v][q] += __shfl_xor_sync(kAll, acc[v][q], off);
+      }
+      if (team == 0) {
+        float* prow = a.partial + (int64_t)k * a.ldp;
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          const int vi = tl + v * TL;
+          if (vi < a.nvec) store_f32<V>(prow + vi * V, acc[v]);
         }
-      } else {
-        for (int k = c0; k < a.n_chunks && a.chunk_item[k] == (int)item; ++k) {
+      }
+      __syncwarp();
+      if (lane == 0) st_release(a.chunk_flag + k, epoch);
+    }
+  }
+  const unsigned lists = teams < 4u ? teams : 4u;  // a group: lists a warp takes at once
+  const int ps = teams > 4u ? __ffs((int)teams) - 3 : 0;  // log2 of the teams per list
+  const int parts = 1 << ps;
+  const int list = team >> ps, part = team & (parts - 1);
+  const unsigned wq = threadIdx.x >> 5;
+  unsigned pend = 0;
+  if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+  auto next_group = [&]() -> unsigned {
+    const unsigned g = (__shfl_sync(kAll, pend, 0) * kClaimQueues + wq) * lists;
+    if (g >= n) return n;  // the claim stays pending: every later call ends here too
+    if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+    return g;
+  };
+  // this team's run [from, from + len) of a list of w entries
+  auto part_of = [&](int w, int& from, int& len) {
+    w = w > 0 ? w : 0;
+    const int run = (w + parts - 1) >> ps;
+    from = part * run < w ? part * run : w;
+    len = w - from < run ? w - from : run;
+  };
+  unsigned g0 = next_group();
+  if (g0 < n) {
+    unsigned g1 = next_group();
+    int4 m0 = __ldg(a.meta + g0 + list), m1 = __ldg(a.meta + g1 + list);
+    int from0, len0;
+    part_of(m0.w, from0, len0);
+    uint32_t e0 = tl < len0 ? __ldg(a.ent + (uint32_t)m0.z + from0 + tl) : 0u;
+    while (g0 < n) {
+      const float s0 = tl < len0 ? dual_scale(e0, scale_g, a.mult) : 0.f;
+      int from1, len1;
+      uint32_t e1 = 0;
+      float acc[VPL][V];
+#pragma unroll
+      for (int v = 0; v < VPL; ++v)
+#pragma unroll
+        for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
+      gather_dual_row<GT, VPL, V, TLC>(acc, lg, lh, a.ent + (uint32_t)m0.z + from0, len0,
+                                       __reduce_max_sync(kAll, len0), e0, s0, scale_g, a.mult, tl, TL, [&] {
+                                         part_of(m1.w, from1, len1);
+                                         if (tl < len1) e1 = __ldg(a.ent + (uint32_t)m1.z + from1 + tl);
+                                       });
+      for (int off = TL; off < TL * parts; off <<= 1) {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+#pragma unroll
+          for (int q = 0; q < V; ++q) acc[v][q] += __shfl_xor_sync(kAll, acc[v][q], off);
+      }
+      if (part == 0 && g0 + list < n) {
+        for (int k = m0.z, ke = m0.z - m0.w; k < ke && m0.w < 0; ++k) {
           if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
           const float* prow = a.partial + (int64_t)k * a.ldp;
 #pragma unroll
@@ -2085,26 +2272,33 @@ __global__ void __launch_bounds__(kThreads) tr_kernel(const TrArgs a) {
             }
           }
         }
-      }
-      // an empty column contributes nothing; do not scale it (m may be inf there)
-      const bool empty = c0 < 0 && a.ptr[item] == a.ptr[item + 1];
-      const float so = (a.scale_out && !empty) ? __ldg(a.mult + item) : 1.f;
-      DT* drow = static_cast<DT*>(a.dx) + (int64_t)item * a.lddx;
+        // an empty column contributes nothing; do not scale it (m may be inf there)
+        const bool scaled = a.scale_out && m0.w != 0;
+        const float so = scaled ? __ldg(a.mult + m0.x) : 1.f;
+        DT* drow = static_cast<DT*>(a.dx) + row_off(m0.x, a.lddx);
 #pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        const int vi = tl + v * TL;
-        if (writer && vi < a.nvec) {
-          if (a.scale_out) {
+        for (int v = 0; v < VPL; ++v) {
+          const int vi = tl + v * TL;
+          if (vi < a.nvec) {
+            if (scaled) {
 #pragma unroll
-            for (int q = 0; q < V; ++q) acc[v][q] = __fmul_rn(acc[v][q], so);
+              for (int q = 0; q < V; ++q) acc[v][q] = __fmul_rn(acc[v][q], so);
+            }
+            store_vec<DT, V>(drow + (int64_t)vi * V, acc[v]);
           }
-          store_vec<DT, V>(drow + (int64_t)vi * V, acc[v]);
         }
       }
+      __syncwarp();
+      g0 = g1;
+      m0 = m1;
+      e0 = e1;
+      from0 = from1;
+      len0 = len1;
+      g1 = next_group();
+      m1 = __ldg(a.meta + g1 + list);
     }
-    __syncwarp();
   }
-  finish_block(a.qs, epoch);
+  finish_block(a.qs, epoch, true, a.claims);
 }
 
 }  // namespace cbm

@@ -47,10 +47,16 @@ template <typename XT, typename YT, int VPL, int V, int FORM>
 int launch_fwd_t(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
   // full-warp teams have their own instantiation (also where X's rows lie 2^32
   // bytes apart or more: that one has 32-bit row strides)
-  static GridCache cache[2];
-  const bool full = a.team == 32 && (uint64_t)a.ldx * sizeof(XT) <= 0xffffffffull;
-  auto kern = full ? fwd_kernel<XT, YT, VPL, V, FORM, 32> : fwd_kernel<XT, YT, VPL, V, FORM, 0>;
-  const int grid = cached_grid(cache[full ? 1 : 0], kern, P->device, kThreads, 0);
+  static GridCache cache[3];
+  int form = a.team == 32 && (uint64_t)a.ldx * sizeof(XT) <= 0xffffffffull ? 1 : 0;
+  auto kern = form == 1 ? fwd_kernel<XT, YT, VPL, V, FORM, 32> : fwd_kernel<XT, YT, VPL, V, FORM, kTeamAny>;
+  if constexpr (VPL == 1) {
+    if (a.team <= 2) {
+      form = 2;
+      kern = fwd_kernel<XT, YT, VPL, V, FORM, kTeamNarrow>;
+    }
+  }
+  const int grid = cached_grid(cache[form], kern, P->device, kThreads, 0);
   if (grid <= 0) return CBM_ERR_CUDA;
   kern<<<grid, kThreads, 0, st>>>(a);
   P->launches++;
@@ -152,11 +158,17 @@ int launch_rev_t(cbm_plan* P, const RevArgs& a, cudaStream_t st) {
   return cuda_status(cudaGetLastError());
 }
 
-template <typename GT, typename DT, int VPL, int V, bool SPLIT = false>
+template <typename GT, typename DT, int VPL, int V>
 int launch_tr_t(cbm_plan* P, const TrArgs& a, cudaStream_t st) {
-  static GridCache cache;
-  auto kern = tr_kernel<GT, DT, VPL, V, SPLIT>;
-  const int grid = cached_grid(cache, kern, P->device, kThreads, 0);
+  static GridCache cache[3];
+  int form = 0;
+  auto kern = tr_kernel<GT, DT, VPL, V, 32>;
+  if constexpr (VPL == 1) {
+    form = a.team == 32 ? 0 : a.team > 2 ? 1 : 2;
+    if (form == 1) kern = tr_kernel<GT, DT, VPL, V, kTeamAny>;
+    if (form == 2) kern = tr_kernel<GT, DT, VPL, V, kTeamNarrow>;
+  }
+  const int grid = cached_grid(cache[form], kern, P->device, kThreads, 0);
   if (grid <= 0) return CBM_ERR_CUDA;
   kern<<<grid, kThreads, 0, st>>>(a);
   P->launches++;

@@ -14,6 +14,6 @@ int launch_rev_v(cbm_plan* P, const RevArgs& a, int vpl, cudaStream_t st) {
 
 int launch_rev(cbm_plan* P, const RevArgs& a, int32_t gdt, bool vec, int vpl, cudaStream_t st) {
   if (gdt == CBM_F32) return vec ? launch_rev_v<float, 4>(P, a, vpl, st) : launch_rev_v<float, 1>(P, a, vpl, st);
-  return vec ? launch_rev_v<__nv_bfloat16, 8>(P, a, vpl, st) : launch_rev_v<__nv_bfloat16, 1>(P, a, vpl, st);
+  return vec ? launch_rev_v<__nv_bfloat16, 4>(P, a, vpl, st) : launch_rev_v<__nv_bfloat16, 1>(P, a, vpl, st);
 }
 }  // namespace cbm

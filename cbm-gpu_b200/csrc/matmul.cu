@@ -191,24 +191,33 @@ int zeros_u32(unsigned** dst, int64_t n, cudaStream_t st, std::vector<void*>& ow
 int rebuild_adjoint_chunks(cbm_plan* P, cudaStream_t st) {
   if (!P->adj_built) return CBM_OK;
   free_all(P->adj_chunk_bufs);
-  std::vector<int32_t> chunk0(P->n_cols, -1), citem;
   std::vector<int64_t> cbeg, cend;
   const int64_t T = P->chunk_nnz;
-  for (int64_t j = 0; j < P->n_cols; ++j) {
-    const int64_t b = P->h_t_ptr[j], e = P->h_t_ptr[j + 1];
-    if (e - b > T) {
-      chunk0[j] = (int32_t)citem.size();
-      for (int64_t s = b; s < e; s += T) {
-        citem.push_back((int32_t)j);
+  // items: the columns by the entry groups of 4 their team steps through,
+  // longest first, so that the lists that share a warp are of like length and
+  // the last ones are short (a split list only adds its chunks' sums)
+  auto entries = [&](int64_t j) { return P->h_t_ptr[j + 1] - P->h_t_ptr[j]; };
+  auto cost = [&](int64_t j) { return entries(j) > T ? (int64_t)1 : (entries(j) + 3) / 4; };
+  std::vector<int64_t> start(T / 4 + 3, 0);
+  for (int64_t j = 0; j < P->n_cols; ++j) start[cost(j) + 1]++;
+  for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
+  std::vector<int4> meta(P->n_cols + kMetaPad, make_int4(0, 0, 0, 0));
+  for (int64_t j = P->n_cols - 1; j >= 0; --j) {
+    int4 m = make_int4((int32_t)j, 0, (int32_t)P->h_t_ptr[j], (int32_t)entries(j));
+    if (entries(j) > T) {
+      const int64_t e = P->h_t_ptr[j + 1];
+      m.z = (int32_t)cbeg.size();
+      for (int64_t s = P->h_t_ptr[j]; s < e; s += T) {
         cbeg.push_back(s);
         cend.push_back(std::min(e, s + T));
       }
+      m.w = m.z - (int32_t)cbeg.size();
     }
+    meta[P->n_cols - 1 - start[cost(j)]++] = m;
   }
-  P->n_t_chunks = (int64_t)citem.size();
+  P->n_t_chunks = (int64_t)cbeg.size();
   int rc;
-  if ((rc = upload(&P->d_t_chunk0, chunk0, st, P->adj_chunk_bufs))) return rc;
-  if ((rc = upload(&P->d_t_chunk_item, citem, st, P->adj_chunk_bufs))) return rc;
+  if ((rc = upload(&P->d_t_meta, meta, st, P->adj_chunk_bufs))) return rc;
   if ((rc = upload(&P->d_t_chunk_beg, cbeg, st, P->adj_chunk_bufs))) return rc;
   if ((rc = upload(&P->d_t_chunk_end, cend, st, P->adj_chunk_bufs))) return rc;
   if ((rc = zeros_u32(&P->d_t_chunk_flag, P->n_t_chunks, st, P->adj_chunk_bufs))) return rc;
@@ -237,8 +246,7 @@ int build_adjoint(cbm_plan* P, cudaStream_t st) {
   // internal nodes in reverse item (level) order; a children list longer than
   // kRevChunk is summed in chunk items queued just before its node
   constexpr int64_t kRevChunk = 64;
-  std::vector<int32_t> rnode, rslot, rchunk0, rnchunk;
-  std::vector<int64_t> rptr(1, 0);
+  std::vector<int4> meta;
   std::vector<uint32_t> rent;
   int32_t n_rev_chunks = 0;
   for (int64_t i = n - 1; i >= 0; --i) {
@@ -247,32 +255,24 @@ int build_adjoint(cbm_plan* P, cudaStream_t st) {
     const int64_t nk = cptr[w + 1] - cptr[w];
     const bool split = nk > kRevChunk;
     const int32_t first = n_rev_chunks;
+    int32_t beg = (int32_t)rent.size();
     for (int64_t k = cptr[w]; k < cptr[w + 1]; ++k) {
       const int32_t c = kids[k];
       rent.push_back(P->h_slot[c] >= 0 ? ((uint32_t)P->h_slot[c] | kInternalBit) : (uint32_t)c);
       if (split && ((k - cptr[w] + 1) % kRevChunk == 0 || k + 1 == cptr[w + 1])) {
-        rnode.push_back(-1);  // chunk item
-        rslot.push_back(n_rev_chunks++);
-        rchunk0.push_back(-1);
-        rnchunk.push_back(0);
-        rptr.push_back((int64_t)rent.size());
+        meta.push_back(make_int4(-1, n_rev_chunks++, beg, (int32_t)rent.size() - beg));  // chunk item
+        beg = (int32_t)rent.size();
       }
     }
-    rnode.push_back(w);
-    rslot.push_back(P->h_slot[w]);
-    rchunk0.push_back(split ? first : -1);
-    rnchunk.push_back(split ? n_rev_chunks - first : 0);
-    rptr.push_back((int64_t)rent.size());  // empty range when split
+    meta.push_back(split ? make_int4(w, P->h_slot[w], first, first - n_rev_chunks)
+                         : make_int4(w, P->h_slot[w], beg, (int32_t)nk));
   }
-  P->n_rev_items = (int64_t)rnode.size();
+  P->n_rev_items = (int64_t)meta.size();
   P->n_rev_chunks = n_rev_chunks;
+  meta.resize(meta.size() + kMetaPad, make_int4(-1, 0, 0, 0));
   int rc;
-  if ((rc = upload(&P->d_rev_node, rnode, st, P->adj_bufs))) return rc;
-  if ((rc = upload(&P->d_rev_chunk0, rchunk0, st, P->adj_bufs))) return rc;
-  if ((rc = upload(&P->d_rev_nchunk, rnchunk, st, P->adj_bufs))) return rc;
+  if ((rc = upload(&P->d_rev_meta, meta, st, P->adj_bufs))) return rc;
   if ((rc = zeros_u32(&P->d_rev_chunk_flag, n_rev_chunks, st, P->adj_bufs))) return rc;
-  if ((rc = upload(&P->d_rev_slot, rslot, st, P->adj_bufs))) return rc;
-  if ((rc = upload(&P->d_rev_ptr, rptr, st, P->adj_bufs))) return rc;
   if ((rc = upload(&P->d_rev_ent, rent, st, P->adj_bufs))) return rc;
   if ((rc = zeros_u32(&P->d_adj_flag, P->n_internal, st, P->adj_bufs))) return rc;
   // transposed delta: column j lists (row v or its slot, sign), sorted on the GPU
@@ -702,7 +702,12 @@ int cbm_matmul_adjoint(cbm_plan* P, int32_t op, const void* g, int32_t gdt, int6
   const bool need_ws = P->n_internal > 0 || P->n_t_chunks > 0;
   if (need_ws && (!ws || ws_bytes < need)) return CBM_ERR_WORKSPACE;
   if (ws && reinterpret_cast<uintptr_t>(ws) % 16 != 0) return CBM_ERR_INVALID;
-  const Shape sh = pick_shape(gdt, ddt, g, ldg, dx, lddx, n_cols);
+  Shape sh = pick_shape(gdt, ddt, g, ldg, dx, lddx, n_cols);
+  if (sh.vec) {
+    // vectors of four elements in both types: H's rows are FP32
+    sh.v = 4;
+    sh.cb = block_cols(4);
+  }
   for (int64_t c0 = 0; c0 < n_cols; c0 += sh.cb) {
     const int64_t cols = std::min(sh.cb, n_cols - c0);
     const int64_t nvec = cols / sh.v;
@@ -717,16 +722,13 @@ int cbm_matmul_adjoint(cbm_plan* P, int32_t op, const void* g, int32_t gdt, int6
       RevArgs r;
       std::memset(&r, 0, sizeof(r));
       r.n_items = (int32_t)P->n_rev_items;
-      r.node = P->d_rev_node;
-      r.slot = P->d_rev_slot;
-      r.ptr = P->d_rev_ptr;
+      r.meta = P->d_rev_meta;
       r.ent = P->d_rev_ent;
-      r.chunk0 = P->d_rev_chunk0;
-      r.nchunk = P->d_rev_nchunk;
       r.mult = P->d_mult;
       r.scale_g = op == CBM_OP_DADX;
       r.flag = P->d_adj_flag;
       r.chunk_flag = P->d_rev_chunk_flag;
+      r.claims = P->d_claims;
       r.partial = rpartial;
       r.qs = P->d_qs;
       r.g = gb;
@@ -735,24 +737,19 @@ int cbm_matmul_adjoint(cbm_plan* P, int32_t op, const void* g, int32_t gdt, int6
       r.ldp = (int32_t)ldp;
       r.nvec = (int32_t)nvec;
       r.team = team;
-      // every reverse item waits on its children, claimed just before it: one
-      // item per claim keeps a wait from holding up the claim's other items
-      // (measured on the 170K-node GCN graph: 0.42 -> 0.26 ms at 40 columns)
-      r.rows_per_claim = 1;
       r.timeout_ns = P->timeout_ns;
       if ((rc = launch_rev(P, r, gdt, sh.vec, vpl, st))) return rc;
     }
     TrArgs t;
     std::memset(&t, 0, sizeof(t));
     t.n_items = (int32_t)P->n_cols;
-    t.ptr = P->d_t_ptr;
+    t.meta = P->d_t_meta;
     t.ent = P->d_t_ent;
     t.n_chunks = (int32_t)P->n_t_chunks;
-    t.chunk0 = P->d_t_chunk0;
-    t.chunk_item = P->d_t_chunk_item;
     t.chunk_beg = P->d_t_chunk_beg;
     t.chunk_end = P->d_t_chunk_end;
     t.chunk_flag = P->d_t_chunk_flag;
+    t.claims = P->d_claims;
     t.mult = P->d_mult;
     t.scale_g = op == CBM_OP_DADX;
     t.scale_out = op == CBM_OP_ADX || op == CBM_OP_DADX;
@@ -766,7 +763,6 @@ int cbm_matmul_adjoint(cbm_plan* P, int32_t op, const void* g, int32_t gdt, int6
     t.nvec = (int32_t)nvec;
     t.partial = partial;
     t.team = team;
-    t.rows_per_claim = claim_rows(P);
     t.timeout_ns = P->timeout_ns;
     if ((rc = launch_tr(P, t, gdt, ddt, sh.vec, vpl, st))) return rc;
   }

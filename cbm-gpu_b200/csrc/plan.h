@@ -93,20 +93,15 @@ struct cbm_plan {
   // adjoint layout (built on first use)
   bool adj_built = false;
   int64_t n_rev_items = 0, n_rev_chunks = 0;
-  int32_t* d_rev_chunk0 = nullptr;
-  int32_t* d_rev_nchunk = nullptr;
   unsigned* d_rev_chunk_flag = nullptr;
-  int32_t* d_rev_node = nullptr;   // internal nodes (and chunk items), deepest level first
-  int32_t* d_rev_slot = nullptr;
-  int64_t* d_rev_ptr = nullptr;    // children lists
+  int4* d_rev_meta = nullptr;      // one record per item (RevArgs), deepest level first
   uint32_t* d_rev_ent = nullptr;   // child | internal << 30 (slot if internal)
   unsigned* d_adj_flag = nullptr;  // [n_internal]
   std::vector<int64_t> h_t_ptr;    // transposed delta: entries per column
   int64_t* d_t_ptr = nullptr;
   uint32_t* d_t_ent = nullptr;     // row (or slot) | internal << 30 | sign << 31
   int64_t n_t_chunks = 0;
-  int32_t* d_t_chunk0 = nullptr;
-  int32_t* d_t_chunk_item = nullptr;
+  int4* d_t_meta = nullptr;        // one record per column, longest lists first (TrArgs)
   int64_t* d_t_chunk_beg = nullptr;
   int64_t* d_t_chunk_end = nullptr;
   unsigned* d_t_chunk_flag = nullptr;

@@ -187,3 +187,35 @@ def test_rows_of_x_4_gib_apart(cols):
     top = xs[0] + xs[1]
     assert torch.equal(y.cpu(), torch.stack([top, -xs[1] + top]))
     p.check_device()
+
+
+@pytest.mark.parametrize("op", ["ax", "dadx"])
+@pytest.mark.parametrize("chunk", [32, 256])
+@pytest.mark.parametrize("dtype,cols", [(torch.float32, c) for c in (1, 3, 4, 8, 12, 16, 20, 33, 40, 64, 128, 132, 256,
+                                                                     300, 1028)] +
+                         [(torch.bfloat16, c) for c in (1, 5, 8, 16, 24, 40, 128, 136, 520, 1032)])
+def test_adjoint_of_a_deep_tree(op, chunk, dtype, cols):
+    """dX = M Delta^T P^T M G against FP64, within the bound of any summation
+    order: 2 * terms * 2^-24 of the magnitudes summed (+ 3 scalings)."""
+    s = _deep_structure(seed=5)
+    n, crow, col, sign, br, src, dst, mult = s
+    p = _plan(s)
+    p.tune(chunk_nnz=chunk)
+    g = torch.randn(n, cols, device="cuda").to(dtype)
+    dx = torch.full((n, cols), float("nan"), device="cuda")
+    p.adjoint(op, g, dx)
+    m = mult.astype(np.float64) if op == "dadx" else np.ones(n)
+    h = g.double().cpu().numpy() * m[:, None]
+    mag, terms = np.abs(h), np.ones(n)
+    for u, v in zip(src[::-1], dst[::-1]):  # deepest first: children into parents
+        h[u] += h[v]
+        mag[u] += mag[v]
+        terms[u] += terms[v]
+    rows = np.repeat(np.arange(n), np.diff(crow))
+    exact, total, count = np.zeros((n, cols)), np.zeros((n, cols)), np.zeros(n)
+    np.add.at(exact, col, sign[:, None].astype(np.float64) * h[rows])
+    np.add.at(total, col, mag[rows])
+    np.add.at(count, col, 1 + terms[rows])
+    err = np.abs(dx.double().cpu().numpy() - exact * m[:, None])
+    assert (err <= 2.0 * (count[:, None] + 3) * 2.0 ** -24 * total * m[:, None] + 1e-30).all()
+    p.check_device()
