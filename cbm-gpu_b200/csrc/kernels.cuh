@@ -58,7 +58,11 @@ struct QueueState {
 struct FwdArgs {
   // rows in level order
   int32_t n_items;
-  const int4* meta;          // register kernel: one record per item (kernels below)
+  // register kernel: one record per item (layout at the kernel) and the items'
+  // slots, in record order (level by level, as the items)
+  const int4* meta;
+  const int32_t* rec_self_slot;
+  const int32_t* rec_par_slot;
   const int32_t* node;       // node id per item; bit 31 set: node has children
   const int64_t* ptr;        // [n_items + 1]
   const uint32_t* ent;       // column | sign << 31
@@ -753,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
       auto load_parent = [&]() {
         const float* src;
         if (state) {
-          src = a.pstate + (int64_t)__ldg(a.par_slot + item) * a.ldp;
+          src = a.pstate + (int64_t)__ldg(a.rec_par_slot + item) * a.ldp;
         } else {
           src = static_cast<const float*>(a.y) + row_off(p, a.ldy);
         }
@@ -852,7 +856,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
                   // the rounding errors (of the ratio's product and quotient too)
                   float rp[V];
                   if (cread) {
-                    load_f32_cg<V>(a.pcomp + (int64_t)__ldg(a.par_slot + item) * a.ldp + vi * V, rp);
+                    load_f32_cg<V>(a.pcomp + (int64_t)__ldg(a.rec_par_slot + item) * a.ldp + vi * V, rp);
                   } else {
 #pragma unroll
                     for (int q = 0; q < V; ++q) rp[q] = 0.f;
@@ -884,7 +888,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
             }
           }
           const bool keep = m0.x < 0 && !a.skip_parent;  // children read this row
-          const int ss = keep && (state || COMP) ? __ldg(a.self_slot + item) : 0;
+          const int ss = keep && (state || COMP) ? __ldg(a.rec_self_slot + item) : 0;
           if (COMP && cmode) {
             // the row's value is acc + cres, rounded once; its residual is kept for
             // the children of an internal node

@@ -368,7 +368,10 @@ int cbm_plan_debug_set_parent(cbm_plan* P, int64_t item, int32_t parent_node, vo
   P->h_item_par[item] = parent_node;
   P->h_item_par_item[item] = par_item;
   const int32_t rec[2] = {record_node(P, item), parent_node};
-  if (cudaMemcpyAsync(reinterpret_cast<char*>(P->d_meta + item), rec, sizeof(rec), cudaMemcpyHostToDevice, st) !=
+  if (cudaMemcpyAsync(reinterpret_cast<char*>(P->d_meta + P->h_rec[item]), rec, sizeof(rec), cudaMemcpyHostToDevice,
+                      st) != cudaSuccess)
+    return CBM_ERR_CUDA;
+  if (cudaMemcpyAsync(P->d_rec_par_slot + P->h_rec[item], &zero, sizeof(int32_t), cudaMemcpyHostToDevice, st) !=
       cudaSuccess)
     return CBM_ERR_CUDA;
   if (cudaMemcpyAsync(P->d_par_item + item, &par_item, sizeof(int32_t), cudaMemcpyHostToDevice, st) != cudaSuccess)
@@ -442,6 +445,8 @@ int matmul_impl(cbm_plan* P, int32_t op, float gin_scale, const void* x, int32_t
     std::memset(&a, 0, sizeof(a));
     a.n_items = (int32_t)P->n_items;
     a.meta = P->d_meta;
+    a.rec_self_slot = P->d_rec_self_slot;
+    a.rec_par_slot = P->d_rec_par_slot;
     a.sval = P->d_sval;
     a.csval = P->d_csval;
     a.node = P->d_node;

@@ -51,10 +51,13 @@ struct cbm_plan {
 
   std::vector<int32_t> h_item_par;       // parent node per item, as on the device
   std::vector<int32_t> h_item_par_item;  // its queue position, -1
+  std::vector<int32_t> h_rec;            // the register kernel's record of each item
 
   // forward layout (device); d_ptr/d_ent/d_val and d_cent/d_cval are the
   // stream layout rebuilt with the chunk size (build_layout)
-  int4* d_meta = nullptr;       // one 16-byte record per item (kernels.cuh, item_meta)
+  int4* d_meta = nullptr;       // the register kernel's records, 16 bytes per item
+  int32_t* d_rec_self_slot = nullptr;  // d_self_slot and d_par_slot in record order
+  int32_t* d_rec_par_slot = nullptr;
   float* d_sval = nullptr;      // s * m[col] per entry of d_ent / d_cent, once the plan has
   float* d_csval = nullptr;     // multipliers (square A, values +-1; null: formed in the kernel)
   int32_t* d_node = nullptr;
@@ -135,6 +138,7 @@ namespace cbm {
 int cuda_status(cudaError_t e);
 void free_all(std::vector<void*>& v);
 int build_layout(cbm_plan* P, cudaStream_t st);
+int build_records(cbm_plan* P, const std::vector<int64_t>& first, const std::vector<int32_t>& chunk0, cudaStream_t st);
 int scale_entries(cbm_plan* P, cudaStream_t st);
 int32_t record_node(const cbm_plan* P, int64_t item);
 int build_units(cbm_plan* P, cudaStream_t st);

@@ -14,16 +14,17 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _deep_structure(n=700, seed=0):
-    """A forest with most rows below level 0: many parents directly precede
-    their child, and about a tenth of the rows are 32 entries or longer."""
+def _deep_structure(n=700, seed=0, near=0.45, child=0.9):
+    """A forest in which a share `near` of the rows hangs from one of the three
+    rows before it and a share `child` from any earlier row (most rows are below
+    level 0 by default); about a tenth of the rows are 32 entries or longer."""
     rng = np.random.default_rng(seed)
     parent = np.full(n, -1)
     for v in range(1, n):
         u = rng.random()
-        if u < 0.45:
+        if u < near:
             parent[v] = v - 1 - rng.integers(0, min(v, 3))
-        elif u < 0.9:
+        elif u < child:
             parent[v] = rng.integers(0, v)
     depth = np.zeros(n, dtype=int)
     for v in range(n):
@@ -77,6 +78,31 @@ def test_deep_tree_matches_oracle(op, dtype, cols):
     if dtype == torch.bfloat16:
         yb = torch.empty(s[0], cols, device="cuda", dtype=dtype)
         p.matmul(op, x, yb)
+        assert torch.equal(yb.cpu(), torch.from_numpy(ref).to(dtype))
+    p.check_device()
+
+
+@pytest.mark.parametrize("dtype,cols", [(torch.float32, 1), (torch.float32, 12), (torch.float32, 33),
+                                        (torch.float32, 128), (torch.bfloat16, 40), (torch.bfloat16, 128)])
+def test_shallow_tree_matches_oracle(dtype, cols):
+    """Records in length order inside windows (two windows in level 0 here)."""
+    from oracle import oracle
+
+    s = _deep_structure(n=11000, seed=6, near=0.1, child=0.2)
+    n, crow, col, sign, br, src, dst, _ = s
+    p = _plan(s)
+    p.tune(variant="register")
+    x = torch.randn(n, cols, device="cuda").to(dtype)
+    xn = x.float().cpu().numpy()
+    y = torch.full((n, cols), float("nan"), device="cuda")
+    p.matmul("dadx", x, y)
+    ref = _oracle("dadx", s, xn)
+    np.testing.assert_array_equal(y.cpu().numpy(), ref)
+    p.matmul_gin(x, y, 0.25)
+    np.testing.assert_array_equal(y.cpu().numpy(), oracle.spmm_update_add(crow, col, sign, xn, 0.25, br, src, dst))
+    if dtype == torch.bfloat16:
+        yb = torch.empty(n, cols, device="cuda", dtype=dtype)
+        p.matmul("dadx", x, yb)
         assert torch.equal(yb.cpu(), torch.from_numpy(ref).to(dtype))
     p.check_device()
 
