@@ -371,6 +371,11 @@ __host__ __device__ constexpr int reg_in_flight() {
   const int u = (VPL >= 4 ? 32 : 16) / (VPL * Raw<XT, V>::regs);
   return u < 1 ? 1 : (u > 8 ? 8 : u);
 }
+// The same where a plan has so few rows that a warp gets one group of them at
+// most (FORM_FEW): occupancy then buys nothing, and a row of 30 entries is four
+// exposed round trips instead of eight (4,096 nodes, 64 FP32 columns: 16.5 -> 12.2 us on
+// the device; 128 BF16 columns 23.9 -> 17.8, 4,000 nodes and 47 columns 47 -> 38).
+constexpr int kFewInFlight = 8;
 
 // Entry idx's scale before the row factor: s, the stored value, or s * m[col]
 // (from the plan's array when it has one).
@@ -424,12 +429,11 @@ constexpr int kTeamNarrow = 1;
 // ahead.  `between` runs once, after the first group's gathers are issued and
 // before anything waits for them: the place for loads the next row needs, and
 // for an acquire, whose latency then hides under the gathers'.
-template <typename XT, int VPL, int V, int TLC, bool WIDE, typename Between>
+template <typename XT, int VPL, int V, int TLC, int U, bool WIDE, typename Between>
 __device__ __forceinline__ void gather_row(float (&acc)[VPL][V], const Lane<XT, VPL, V, WIDE>& ln,
                                            const uint32_t* __restrict__ ent, const float* __restrict__ vals, int len,
                                            int wlen, uint32_t e, float s, float dv, int scale_mode,
                                            const float* __restrict__ mult, int tl, int team_lanes, Between between) {
-  constexpr int U = reg_in_flight<XT, VPL, V>();
   using R = Raw<XT, V>;
   const int TL = TLC == 32 ? 32 : team_lanes;
   if (wlen <= 0) {
@@ -560,7 +564,7 @@ __device__ __forceinline__ void gather_row(float (&acc)[VPL][V], const Lane<XT, 
 // against 137 with two).
 template <typename XT, typename YT, int VPL, int FORM, int TLC>
 __host__ __device__ constexpr int fwd_min_blocks() {
-  return FORM == 2 || VPL > 4 ? 1 : VPL == 4 ? 2 : VPL == 1 && TLC == 32 ? 4 : 3;
+  return FORM == 2 || VPL > 4 ? 1 : FORM == 3 ? 2 : VPL == 4 ? 2 : VPL == 1 && TLC == 32 ? 4 : 3;
 }
 
 // s + e == a + b exactly (Knuth's TwoSum; explicit roundings, no contraction)
@@ -633,13 +637,15 @@ constexpr int kMetaPad = 32;
 constexpr int kPreMark = INT_MIN;
 
 // What a register-kernel instantiation leaves out: FORM_PLAIN has no GIN term
-// and no compensation.
-enum RowForm : int { FORM_PLAIN = 0, FORM_GIN = 1, FORM_COMP = 2 };
+// and no compensation, nor has FORM_FEW, which keeps more gathers in flight.
+enum RowForm : int { FORM_PLAIN = 0, FORM_GIN = 1, FORM_COMP = 2, FORM_FEW = 3 };
 
 template <typename XT, typename YT, int VPL, int V, int FORM, int TLC>
 __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, TLC>())) fwd_kernel(const FwdArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr bool COMP = FORM == FORM_COMP;
+  constexpr bool kPlain = FORM == FORM_PLAIN || FORM == FORM_FEW;
+  constexpr int U = FORM == FORM_FEW ? kFewInFlight : reg_in_flight<XT, VPL, V>();
   // parents' rows come from the FP32 state rows
   const bool state = sizeof(YT) != 4 || FORM == FORM_GIN || (COMP && a.gin);
   const int lane = threadIdx.x & 31;
@@ -703,7 +709,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
       for (int v = 0; v < VPL; ++v)
 #pragma unroll
         for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-      gather_row<XT, VPL, V, TLC>(acc, ln, ent, cv, len, TLC == 32 ? len : __reduce_max_sync(kAll, len), e, s, dv,
+      gather_row<XT, VPL, V, TLC, U>(acc, ln, ent, cv, len, TLC == 32 ? len : __reduce_max_sync(kAll, len), e, s, dv,
                                   a.scale_mode, a.mult, tl, TL, [] {});
       if (have) {
 #pragma unroll
@@ -733,8 +739,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
   };
   unsigned g0 = next_group();
   if (g0 < n) {
-    unsigned g1 = next_group();
-    int4 m0 = __ldg(a.meta + g0 + team), m1 = __ldg(a.meta + g1 + team);
+    int4 m0 = __ldg(a.meta + g0 + team);
     uint32_t e0 = 0;
     float s0 = 0.f;
     unsigned f0 = 0;
@@ -742,6 +747,8 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
       e0 = __ldg(a.ent + (uint32_t)m0.z + tl);
       s0 = reg_scale(e0, vals ? vals + (uint32_t)m0.z : nullptr, tl, a.scale_mode, a.mult);
     }
+    unsigned g1 = next_group();
+    int4 m1 = __ldg(a.meta + g1 + team);
     if (a.skip_parent) m0.y = -1, m1.y = -1;
     if (m0.y >= 0) f0 = ld_acquire(a.node_flag + m0.y);
     while (g0 < n) {
@@ -779,7 +786,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
       // ahead of the gathers, but for one piece per lane, where those registers
       // are worth more as occupancy (100,000-node GIN, 256 FP32 columns: 198 ->
       // 178 us; 200,000 nodes, 128 columns: 376 -> 353 us the other way)
-      if (FORM != FORM_PLAIN && VPL > 1) load_self();
+      if (!kPlain && VPL > 1) load_self();
       if (ratio && p >= 0) dp = __ldg(a.mult + p);
       float acc[VPL][V];
 #pragma unroll
@@ -790,7 +797,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
       uint32_t e1 = 0;
       float s1 = 0.f;
       unsigned f1 = 0;
-      gather_row<XT, VPL, V, TLC>(acc, ln, a.ent + (uint32_t)m0.z, vals ? vals + (uint32_t)m0.z : nullptr, len,
+      gather_row<XT, VPL, V, TLC, U>(acc, ln, a.ent + (uint32_t)m0.z, vals ? vals + (uint32_t)m0.z : nullptr, len,
                                   TLC == 32 ? len : __reduce_max_sync(kAll, len), e0, s0, drow ? dv : 1.f,
                                   a.scale_mode, a.mult, tl, TL, [&] {
                                     if (tl < m1.w) {
@@ -800,7 +807,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
                                     if (m1.y >= 0) f1 = ld_acquire(a.node_flag + m1.y);
                                   });
 
-      if (FORM != FORM_PLAIN && VPL == 1) load_self();
+      if (!kPlain && VPL == 1) load_self();
 
       // ---- the row's end: chunk partials, parent, store, ready flag
       const int serial = TLC != 32 && __any_sync(kAll, have && (m0.x & kNearBit) != 0) ? (int)teams : 1;
@@ -915,7 +922,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
           for (int v = 0; v < VPL; ++v) {
             const int vi = tl + v * TL;
             if (vi < a.nvec) {
-              if constexpr (FORM == FORM_PLAIN) {
+              if constexpr (kPlain) {
                 store_vec<YT, V>(yrow + (int64_t)vi * V, acc[v]);
               } else {
                 float xs[V], out[V];

@@ -50,7 +50,7 @@ int launch_fwd_t(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
   static GridCache cache[3];
   int form = a.team == 32 && (uint64_t)a.ldx * sizeof(XT) <= 0xffffffffull ? 1 : 0;
   auto kern = form == 1 ? fwd_kernel<XT, YT, VPL, V, FORM, 32> : fwd_kernel<XT, YT, VPL, V, FORM, kTeamAny>;
-  if constexpr (VPL == 1) {
+  if constexpr (VPL == 1 && FORM != FORM_FEW) {
     if (a.team <= 2) {
       form = 2;
       kern = fwd_kernel<XT, YT, VPL, V, FORM, kTeamNarrow>;
@@ -139,6 +139,13 @@ int launch_tma_any(cbm_plan* P, const FwdArgs& a, int team, int vpl, const CUten
 
 template <typename XT, typename YT, int V, int FORM>
 int launch_fwd_v(cbm_plan* P, const FwdArgs& a, int vpl, cudaStream_t st) {
+  // few rows: one group per warp at 16 resident warps per SM (narrower teams are
+  // slower so: 8,000 nodes, 24 BF16 columns 64 -> 71 us)
+  if constexpr (FORM == FORM_PLAIN) {
+    const int64_t groups = ((int64_t)a.n_items * a.team + 31) / 32;
+    if (vpl == 1 && a.team >= 8 && groups <= (int64_t)sm_count(P->device) * 16)
+      return launch_fwd_t<XT, YT, 1, V, FORM_FEW>(P, a, st);
+  }
   switch (vpl) {
     case 1: return launch_fwd_t<XT, YT, 1, V, FORM>(P, a, st);
     case 2: return launch_fwd_t<XT, YT, 2, V, FORM>(P, a, st);

@@ -83,15 +83,19 @@ def test_deep_tree_matches_oracle(op, dtype, cols):
 
 
 @pytest.mark.parametrize("dtype,cols", [(torch.float32, 1), (torch.float32, 12), (torch.float32, 33),
-                                        (torch.float32, 128), (torch.bfloat16, 40), (torch.bfloat16, 128)])
-def test_shallow_tree_matches_oracle(dtype, cols):
-    """Records in length order inside windows (two windows in level 0 here)."""
+                                        (torch.float32, 64), (torch.float32, 128), (torch.bfloat16, 40),
+                                        (torch.bfloat16, 128)])
+@pytest.mark.parametrize("near,child", [(0.1, 0.2), (0.45, 0.9)], ids=["shallow", "deep"])
+def test_larger_trees_match_oracle(near, child, dtype, cols):
+    """More groups than resident warps; on the shallow tree also records in
+    length order inside windows (two of them in level 0)."""
     from oracle import oracle
 
-    s = _deep_structure(n=11000, seed=6, near=0.1, child=0.2)
+    s = _deep_structure(n=11000, seed=6, near=near, child=child)
     n, crow, col, sign, br, src, dst, _ = s
     p = _plan(s)
     p.tune(variant="register")
+    p.set_compensation(-1)
     x = torch.randn(n, cols, device="cuda").to(dtype)
     xn = x.float().cpu().numpy()
     y = torch.full((n, cols), float("nan"), device="cuda")
