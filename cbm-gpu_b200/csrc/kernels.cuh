@@ -188,18 +188,6 @@ struct Vec<float, 1> {
   static __device__ __forceinline__ void load(const float* p, float (&o)[1]) { o[0] = __ldg(p); }
 };
 template <>
-struct Vec<__nv_bfloat16, 8> {
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[8]) {
-    const uint4 t = __ldg(reinterpret_cast<const uint4*>(p));
-    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      o[2 * i] = __uint_as_float(w[i] << 16);
-      o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-    }
-  }
-};
-template <>
 struct Vec<__nv_bfloat16, 4> {
   static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[4]) {
     const uint2 t = __ldg(reinterpret_cast<const uint2*>(p));
