@@ -623,6 +623,10 @@ constexpr int kNodeMask = 0x3fffffff;
 constexpr int kMetaPad = 32;
 // entry count of a presummed row's record
 constexpr int kPreMark = INT_MIN;
+// One past the last chunk of a record (z, w); z itself where the row is not split.
+__host__ __device__ constexpr int chunk_stop(int z, int w) { return w < 0 && w != kPreMark ? z - w : z; }
+static_assert(chunk_stop(INT_MAX, kPreMark) == INT_MAX && chunk_stop(5, 12) == 5 && chunk_stop(5, -3) == 8,
+              "a presummed row's record, whose mark has no negative, walks no chunks");
 
 // What a register-kernel instantiation leaves out: FORM_PLAIN has no GIN term
 // and no compensation, nor has FORM_FEW, which keeps more gathers in flight.
@@ -813,7 +817,7 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
               }
             }
           }
-          for (int k = m0.z, ke = m0.z - m0.w; k < ke && m0.w < 0 && m0.w != kPreMark; ++k) {
+          for (int k = m0.z, ke = chunk_stop(m0.z, m0.w); k < ke; ++k) {
             if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
             const float* prow = a.partial + (int64_t)k * a.ldp;
 #pragma unroll
