@@ -198,6 +198,18 @@ struct Vec<__nv_bfloat16, 4> {
   }
 };
 template <>
+struct Vec<__nv_bfloat16, 8> {
+  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[8]) {
+    const uint4 t = __ldg(reinterpret_cast<const uint4*>(p));
+    const uint32_t w[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      o[2 * i] = __uint_as_float(w[i] << 16);
+      o[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+  }
+};
+template <>
 struct Vec<__nv_bfloat16, 1> {
   static __device__ __forceinline__ void load(const __nv_bfloat16* p, float (&o)[1]) {
     const unsigned short b = __ldg(reinterpret_cast<const unsigned short*>(p));
@@ -1828,14 +1840,18 @@ struct RevArgs {
   long long timeout_ns;
 };
 
+// Entries above which a list is split over all teams of a warp.  Measured above 32, 64
+// and 0 (the chunks then in a phase of their own), 40 FP32 columns: 10,000-node GCN
+// graph 85 us each, 170,000 nodes 169, 168 and 199.
+constexpr int kSoloLen = 64;
+
 struct TrArgs {
-  int32_t n_items;       // columns of Delta
-  const int4* meta;      // per item, longest lists first: x = column, z = first
-                         // entry and w = entries, or first chunk and minus the chunks
+  int32_t n_items;       // chunks of long lists, then the columns of Delta
+  int32_t n_solo;        // of these, the first ones: a warp takes each alone
+  const int4* meta;      // per item, columns longest lists first: x = column, z = first
+                         // entry and w = entries, or first chunk and minus the chunks;
+                         // a chunk's x is ~its number
   const uint32_t* ent;   // row | internal bit (slot then) | sign << 31
-  int32_t n_chunks;
-  const int64_t* chunk_beg;
-  const int64_t* chunk_end;
   unsigned int* chunk_flag;
   unsigned int* claims;  // kClaimQueues counters
   const float* mult;
@@ -2051,15 +2067,16 @@ __device__ __forceinline__ float dual_scale(uint32_t e, bool scale_g, const floa
   return (!scale_g || (e & kInternalBit)) ? sgn : sgn * __ldg(mult + (e & kIndexMask));
 }
 
-// acc += sum of s * (internal ? H[slot] : G[row]) over `len` entries, in order:
-// gather_row (above) with a row source per entry.
-template <typename GT, int VPL, int V, int TLC, typename Between>
-__device__ __forceinline__ void gather_dual_row(float (&acc)[VPL][V], const Lane<GT, VPL, V, true>& lg,
+// sums += sum of s * (internal ? H[slot] : G[row]) over `len` entries, dealt over
+// the S sums in turn: gather_row (above) with a row source per entry.
+template <typename GT, int VPL, int V, int TLC, int S, typename Between>
+__device__ __forceinline__ void gather_dual_row(float (&acc)[S][VPL][V], const Lane<GT, VPL, V, true>& lg,
                                                 const Lane<float, VPL, V, false>& lh,
                                                 const uint32_t* __restrict__ ent, int len, int wlen, uint32_t e,
                                                 float s, bool scale_g, const float* __restrict__ mult, int tl,
                                                 int team_lanes, Between between) {
   constexpr int U = dual_in_flight<GT, VPL, V>();
+  static_assert(S == 1 || U % S == 0, "a group's entries are dealt over the sums");
   using D = Dual<GT, V>;
   const int TL = TLC == 32 ? 32 : team_lanes;
   if (wlen <= 0) {
@@ -2101,7 +2118,7 @@ __device__ __forceinline__ void gather_dual_row(float (&acc)[VPL][V], const Lane
             float t[V];
             D::widen(raw[u][v], in[u], t);
 #pragma unroll
-            for (int k = 0; k < V; ++k) acc[v][k] = fmaf(sc[u], t[k], acc[v][k]);
+            for (int k = 0; k < V; ++k) acc[u % S][v][k] = fmaf(sc[u], t[k], acc[u % S][v][k]);
           }
         }
       }
@@ -2138,7 +2155,7 @@ __device__ __forceinline__ void gather_dual_row(float (&acc)[VPL][V], const Lane
             float t[V];
             D::widen(raw[u][v], (eu[u] & kInternalBit) != 0, t);
 #pragma unroll
-            for (int k = 0; k < V; ++k) acc[v][k] = fmaf(su, t[k], acc[v][k]);
+            for (int k = 0; k < V; ++k) acc[u % S][v][k] = fmaf(su, t[k], acc[u % S][v][k]);
           }
         }
       }
@@ -2149,22 +2166,53 @@ __device__ __forceinline__ void gather_dual_row(float (&acc)[VPL][V], const Lane
   }
 }
 
-// (Measured, the whole adjoint on B200, a column per team or warp with every
-// load in turn -> as here: 170,000-node GCN graph, 40 FP32 columns 224 -> 160
-// us, 128 FP32 302 -> 203, 128 BF16 355 -> 279; 200,000 nodes on a shallow tree,
-// 64 / 256 columns 226 / 545 -> 163 / 416.)
-//
+// Sums a team keeps of its share of a list, the entries dealt over them in turn.
+// Four chains of a quarter of the length where teams share a warp: a list is then
+// split at least as finely as over every team of a warp (170,000-node GCN graph,
+// 40 FP32 columns, error against 64 bits: 8.1e-8 over the warp's two teams, 8.8e-8 by
+// one team in one chain, 7.6e-8 by one team in four).
+template <int TLC>
+__host__ __device__ constexpr int dual_sums() {
+  return TLC == 32 ? 1 : 4;
+}
+template <int VPL, int V, int S>
+__device__ __forceinline__ void add_sums(float (&acc)[VPL][V], const float (&sums)[S][VPL][V]) {
+#pragma unroll
+  for (int v = 0; v < VPL; ++v)
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      if constexpr (S == 4)
+        acc[v][q] = __fadd_rn(__fadd_rn(sums[0][v][q], sums[1][v][q]), __fadd_rn(sums[2][v][q], sums[3][v][q]));
+      else
+        acc[v][q] = sums[0][v][q];
+    }
+}
+
 // The transposed gather, a pipeline like the register forward kernel's: lists
 // of like length share a warp (the items are in length order), the next list's
 // record, entries and claim load under the current one's gathers, and the rows
-// are handed out from eight counters.  Where more than four teams share a warp,
-// it still takes four lists: each is split over its share of the teams, in
-// equal runs whose sums are added by shuffles (no order is kept here, the
-// adjoint is held to FP64), as is every chunk over all of them; the narrowest
-// teams would else walk their longest lists alone.
+// are handed out from eight counters.  A list of more than kSoloLen entries, and a
+// chunk of one that is split, has a warp to itself, in equal runs over its teams
+// whose sums are added by shuffles (no order is kept here, the adjoint is held
+// to FP64).  The others run up to four to a warp, on their share of its teams.
+//
+// The chunks are the queue's first items.  A phase of their own ahead of the
+// lists had some SMs work through several while the longest lists, claimed two
+// ahead, waited behind them (10,000 nodes of mean degree 20, 128 FP32 columns: 67 us
+// with the phase, 52 as items; 10,000-node GCN graph, 40 columns 95 -> 68; 50,000 nodes
+// 113 -> 91).  Progress: every counter hands its chunks out before its lists, and
+// only lists wait.
+//
+// Bound by the chain of gathers of the longest lists on small graphs, by
+// instruction issue on large ones.  Measured on B200, the whole adjoint, a column
+// per team or warp with every load in turn -> as here (us): GCN graph of
+// 170,000 nodes, 40 FP32 columns 222 -> 162, 128 FP32 299 -> 203, 40 / 256 BF16 267 / 501
+// -> 217 / 358; of 10,000 nodes, 40 FP32 columns 80 -> 68, 128 86 -> 71; 200,000 nodes on
+// a shallow tree, 8 / 40 / 128 columns 158 / 226 / 361 -> 85 / 164 / 260.
 template <typename GT, typename DT, int VPL, int V, int TLC>
 __global__ void __launch_bounds__(kThreads, (VPL > 2 ? 1 : VPL == 2 ? 2 : 3)) tr_kernel(const TrArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
+  constexpr int S = dual_sums<TLC>();
   const int lane = threadIdx.x & 31;
   const int TL = TLC == 32 ? 32 : a.team;
   const int tl = lane & (TL - 1);
@@ -2174,94 +2222,73 @@ __global__ void __launch_bounds__(kThreads, (VPL > 2 ? 1 : VPL == 2 ? 2 : 3)) tr
   const Lane<GT, VPL, V, true> lg(a.g, a.ldg, a.nvec, tl, TL);
   const Lane<float, VPL, V, false> lh(a.h, a.ldp, a.nvec, tl, TL);
   const bool scale_g = a.scale_g != 0;
-  const unsigned n = (unsigned)a.n_items;
-  if (a.n_chunks > 0) {
-    unsigned pend = 0;
-    if (lane == 0) pend = atomicAdd(&a.qs->next_chunk, 1u);
-    for (;;) {
-      const unsigned k = __shfl_sync(kAll, pend, 0);
-      if (k >= (unsigned)a.n_chunks) break;
-      if (lane == 0) pend = atomicAdd(&a.qs->next_chunk, 1u);
-      const int all = (int)(a.chunk_end[k] - a.chunk_beg[k]);
-      const int run = (all + (int)teams - 1) >> (__ffs((int)teams) - 1);
-      const int from = team * run < all ? team * run : all;
-      const int len = all - from < run ? all - from : run;
-      const uint32_t* ent = a.ent + a.chunk_beg[k] + from;
-      const uint32_t e = tl < len ? __ldg(ent + tl) : 0u;
-      const float s = tl < len ? dual_scale(e, scale_g, a.mult) : 0.f;
-      float acc[VPL][V];
-#pragma unroll
-      for (int v = 0; v < VPL; ++v)
-#pragma unroll
-        for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-      gather_dual_row<GT, VPL, V, TLC>(acc, lg, lh, ent, len, run, e, s, scale_g, a.mult, tl, TL, [] {});
-      for (int off = TL; off < 32; off <<= 1) {
-#pragma unroll
-        for (int v = 0; v < VPL; ++v)
-#pragma unroll
-          for (int q = 0; q < V; ++q) acc[v][q] += __shfl_xor_sync(kAll, acc[v][q], off);
-      }
-      if (team == 0) {
-        float* prow = a.partial + (int64_t)k * a.ldp;
-#pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const int vi = tl + v * TL;
-          if (vi < a.nvec) store_f32<V>(prow + vi * V, acc[v]);
-        }
-      }
-      __syncwarp();
-      if (lane == 0) st_release(a.chunk_flag + k, epoch);
-    }
-  }
-  const unsigned lists = teams < 4u ? teams : 4u;  // a group: lists a warp takes at once
-  const int ps = teams > 4u ? __ffs((int)teams) - 3 : 0;  // log2 of the teams per list
-  const int parts = 1 << ps;
-  const int list = team >> ps, part = team & (parts - 1);
+  const unsigned n = (unsigned)a.n_items, n_solo = (unsigned)a.n_solo;
+  const unsigned lists = teams < 4u ? teams : 4u;  // lists of a group behind the solo ones
+  const int ps_solo = __ffs((int)teams) - 1;       // log2 of the teams per list: all of them,
+  const int ps_shared = teams > 4u ? __ffs((int)teams) - 3 : 0;  // or the list's share
   const unsigned wq = threadIdx.x >> 5;
   unsigned pend = 0;
-  if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
-  auto next_group = [&]() -> unsigned {
-    const unsigned g = (__shfl_sync(kAll, pend, 0) * kClaimQueues + wq) * lists;
-    if (g >= n) return n;  // the claim stays pending: every later call ends here too
+  auto claim = [&] {
     if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+  };
+  // first item of the warp's next group; n when the queue is exhausted
+  auto next_group = [&]() -> unsigned {
+    unsigned g = __shfl_sync(kAll, pend, 0) * kClaimQueues + wq;
+    if (g > n_solo) g = n_solo + (g - n_solo) * lists;
+    if (g >= n) return n;  // the claim stays pending: every later call ends here too
+    claim();
     return g;
   };
-  // this team's run [from, from + len) of a list of w entries
-  auto part_of = [&](int w, int& from, int& len) {
+  auto split_of = [&](unsigned g) { return g < n_solo ? ps_solo : ps_shared; };
+  // this team's run [from, from + len) of a list of w entries split over 2^ps teams
+  auto part_of = [&](int w, int ps, int& from, int& len) {
     w = w > 0 ? w : 0;
-    const int run = (w + parts - 1) >> ps;
+    const int part = team & ((1 << ps) - 1);
+    const int run = (w + (1 << ps) - 1) >> ps;
     from = part * run < w ? part * run : w;
     len = w - from < run ? w - from : run;
   };
+  claim();
   unsigned g0 = next_group();
   if (g0 < n) {
     unsigned g1 = next_group();
-    int4 m0 = __ldg(a.meta + g0 + list), m1 = __ldg(a.meta + g1 + list);
+    int ps0 = split_of(g0), ps1 = split_of(g1);
+    int4 m0 = __ldg(a.meta + g0 + (team >> ps0)), m1 = __ldg(a.meta + g1 + (team >> ps1));
     int from0, len0;
-    part_of(m0.w, from0, len0);
+    part_of(m0.w, ps0, from0, len0);
     uint32_t e0 = tl < len0 ? __ldg(a.ent + (uint32_t)m0.z + from0 + tl) : 0u;
     while (g0 < n) {
       const float s0 = tl < len0 ? dual_scale(e0, scale_g, a.mult) : 0.f;
       int from1, len1;
       uint32_t e1 = 0;
+      float sums[S][VPL][V] = {};
+      gather_dual_row<GT, VPL, V, TLC, S>(sums, lg, lh, a.ent + (uint32_t)m0.z + from0, len0,
+                                          __reduce_max_sync(kAll, len0), e0, s0, scale_g, a.mult, tl, TL, [&] {
+                                            part_of(m1.w, ps1, from1, len1);
+                                            if (tl < len1) e1 = __ldg(a.ent + (uint32_t)m1.z + from1 + tl);
+                                          });
       float acc[VPL][V];
-#pragma unroll
-      for (int v = 0; v < VPL; ++v)
-#pragma unroll
-        for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-      gather_dual_row<GT, VPL, V, TLC>(acc, lg, lh, a.ent + (uint32_t)m0.z + from0, len0,
-                                       __reduce_max_sync(kAll, len0), e0, s0, scale_g, a.mult, tl, TL, [&] {
-                                         part_of(m1.w, from1, len1);
-                                         if (tl < len1) e1 = __ldg(a.ent + (uint32_t)m1.z + from1 + tl);
-                                       });
-      for (int off = TL; off < TL * parts; off <<= 1) {
+      add_sums<VPL, V>(acc, sums);
+      for (int off = TL; off < TL << ps0; off <<= 1) {
 #pragma unroll
         for (int v = 0; v < VPL; ++v)
 #pragma unroll
           for (int q = 0; q < V; ++q) acc[v][q] += __shfl_xor_sync(kAll, acc[v][q], off);
       }
-      if (part == 0 && g0 + list < n) {
-        for (int k = m0.z, ke = m0.z - m0.w; k < ke && m0.w < 0; ++k) {
+      const bool writer = (team & ((1 << ps0) - 1)) == 0 && g0 + (team >> ps0) < n;
+      if (m0.x < 0) {
+        // a chunk, alone on its warp: its sum, then its ready flag
+        float* prow = a.partial + (int64_t)(~m0.x) * a.ldp;
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          const int vi = tl + v * TL;
+          if (writer && vi < a.nvec) store_f32<V>(prow + vi * V, acc[v]);
+        }
+        // the barrier orders the team's stores before lane 0's release, which carries them
+        __syncwarp();
+        if (lane == 0) st_release(a.chunk_flag + ~m0.x, epoch);
+      } else if (writer) {
+        for (int k = m0.z, ke = chunk_stop(m0.z, m0.w); k < ke; ++k) {
           if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
           const float* prow = a.partial + (int64_t)k * a.ldp;
 #pragma unroll
@@ -2297,8 +2324,10 @@ __global__ void __launch_bounds__(kThreads, (VPL > 2 ? 1 : VPL == 2 ? 2 : 3)) tr
       e0 = e1;
       from0 = from1;
       len0 = len1;
+      ps0 = ps1;
       g1 = next_group();
-      m1 = __ldg(a.meta + g1 + list);
+      ps1 = split_of(g1);
+      m1 = __ldg(a.meta + g1 + (team >> ps1));
     }
   }
   finish_block(a.qs, epoch, true, a.claims);

@@ -205,7 +205,8 @@ int launch_fwd_bf16(cbm_plan* P, const FwdArgs& a, int32_t ydt, bool vec, int vp
 int launch_fwd_comp(cbm_plan* P, const FwdArgs& a, int32_t ydt, bool vec, int vpl, cudaStream_t st);
 // second pass of a two-pass product (FP32 Y)
 int launch_prop(cbm_plan* P, const PropArgs& a, bool vec, int vpl, cudaStream_t st);
-int launch_rev(cbm_plan* P, const RevArgs& a, int32_t gdt, bool vec, int vpl, cudaStream_t st);
+// v: elements per vector of G's rows
+int launch_rev(cbm_plan* P, const RevArgs& a, int32_t gdt, int v, int vpl, cudaStream_t st);
 int launch_tr(cbm_plan* P, const TrArgs& a, int32_t gdt, int32_t ddt, bool vec, int vpl, cudaStream_t st);
 
 }  // namespace cbm

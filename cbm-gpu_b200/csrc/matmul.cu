@@ -191,35 +191,36 @@ int zeros_u32(unsigned** dst, int64_t n, cudaStream_t st, std::vector<void*>& ow
 int rebuild_adjoint_chunks(cbm_plan* P, cudaStream_t st) {
   if (!P->adj_built) return CBM_OK;
   free_all(P->adj_chunk_bufs);
-  std::vector<int64_t> cbeg, cend;
   const int64_t T = P->chunk_nnz;
-  // items: the columns by the entry groups of 4 their team steps through,
-  // longest first, so that the lists that share a warp are of like length and
-  // the last ones are short (a split list only adds its chunks' sums)
+  // items: the chunks of split lists, then the columns by the entry groups of 4
+  // their team steps through, longest first, so that the lists that share a
+  // warp are of like length and the last ones are short (a split list only adds
+  // its chunks' sums)
   auto entries = [&](int64_t j) { return P->h_t_ptr[j + 1] - P->h_t_ptr[j]; };
   auto cost = [&](int64_t j) { return entries(j) > T ? (int64_t)1 : (entries(j) + 3) / 4; };
   std::vector<int64_t> start(T / 4 + 3, 0);
-  for (int64_t j = 0; j < P->n_cols; ++j) start[cost(j) + 1]++;
-  for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
-  std::vector<int4> meta(P->n_cols + kMetaPad, make_int4(0, 0, 0, 0));
-  for (int64_t j = P->n_cols - 1; j >= 0; --j) {
-    int4 m = make_int4((int32_t)j, 0, (int32_t)P->h_t_ptr[j], (int32_t)entries(j));
-    if (entries(j) > T) {
-      const int64_t e = P->h_t_ptr[j + 1];
-      m.z = (int32_t)cbeg.size();
-      for (int64_t s = P->h_t_ptr[j]; s < e; s += T) {
-        cbeg.push_back(s);
-        cend.push_back(std::min(e, s + T));
-      }
-      m.w = m.z - (int32_t)cbeg.size();
-    }
-    meta[P->n_cols - 1 - start[cost(j)]++] = m;
+  std::vector<int4> meta;
+  std::vector<int32_t> chunk0(P->n_cols, -1);
+  int64_t n_solo = 0;
+  for (int64_t j = 0; j < P->n_cols; ++j) {
+    start[cost(j) + 1]++;
+    n_solo += cost(j) > kSoloLen / 4;
+    if (entries(j) <= T) continue;
+    chunk0[j] = (int32_t)meta.size();
+    for (int64_t s = P->h_t_ptr[j], e = P->h_t_ptr[j + 1]; s < e; s += T)
+      meta.push_back(make_int4(~(int32_t)meta.size(), 0, (int32_t)s, (int32_t)std::min(T, e - s)));
   }
-  P->n_t_chunks = (int64_t)cbeg.size();
+  const int64_t n_chunks = (int64_t)meta.size();
+  for (size_t k = 1; k < start.size(); ++k) start[k] += start[k - 1];
+  meta.resize(n_chunks + P->n_cols + kMetaPad, make_int4(0, 0, 0, 0));
+  for (int64_t j = P->n_cols - 1; j >= 0; --j)
+    meta[n_chunks + P->n_cols - 1 - start[cost(j)]++] =
+        chunk0[j] < 0 ? make_int4((int32_t)j, 0, (int32_t)P->h_t_ptr[j], (int32_t)entries(j))
+                      : make_int4((int32_t)j, 0, chunk0[j], -(int32_t)((entries(j) + T - 1) / T));
+  P->n_t_chunks = n_chunks;
+  P->n_t_solo = n_chunks + n_solo;
   int rc;
   if ((rc = upload(&P->d_t_meta, meta, st, P->adj_chunk_bufs))) return rc;
-  if ((rc = upload(&P->d_t_chunk_beg, cbeg, st, P->adj_chunk_bufs))) return rc;
-  if ((rc = upload(&P->d_t_chunk_end, cend, st, P->adj_chunk_bufs))) return rc;
   if ((rc = zeros_u32(&P->d_t_chunk_flag, P->n_t_chunks, st, P->adj_chunk_bufs))) return rc;
   return cuda_status(cudaStreamSynchronize(st));
 }
@@ -709,7 +710,7 @@ int cbm_matmul_adjoint(cbm_plan* P, int32_t op, const void* g, int32_t gdt, int6
   if (ws && reinterpret_cast<uintptr_t>(ws) % 16 != 0) return CBM_ERR_INVALID;
   Shape sh = pick_shape(gdt, ddt, g, ldg, dx, lddx, n_cols);
   if (sh.vec) {
-    // vectors of four elements in both types: H's rows are FP32
+    // the gather reads vectors of four elements in both types: H's rows are FP32
     sh.v = 4;
     sh.cb = block_cols(4);
   }
@@ -740,19 +741,26 @@ int cbm_matmul_adjoint(cbm_plan* P, int32_t op, const void* g, int32_t gdt, int6
       r.ldg = ldg;
       r.h = h;
       r.ldp = (int32_t)ldp;
-      r.nvec = (int32_t)nvec;
-      r.team = team;
+      // BF16 rows of one vector of eight, or of more vectors of four than a warp
+      // has lanes, go up the tree in vectors of eight; the widths between run
+      // faster on twice as many lanes.  The whole adjoint on the GCN graph of 60,000
+      // nodes, vectors of eight / four (us): 8 columns 173 / 212, 16 181 / 143, 40 136 /
+      // 124, 128 179 / 159, 160 190 / 220.
+      const int rv = sh.vec && gdt == CBM_BF16 && (cols == 8 || cols > 128) ? 8 : sh.v;
+      const int64_t rnvec = cols / rv;
+      int rteam, rvpl;
+      team_for(rnvec, &rteam, &rvpl);
+      r.nvec = (int32_t)rnvec;
+      r.team = rteam;
       r.timeout_ns = P->timeout_ns;
-      if ((rc = launch_rev(P, r, gdt, sh.vec, vpl, st))) return rc;
+      if ((rc = launch_rev(P, r, gdt, rv, rvpl, st))) return rc;
     }
     TrArgs t;
     std::memset(&t, 0, sizeof(t));
-    t.n_items = (int32_t)P->n_cols;
+    t.n_items = (int32_t)(P->n_t_chunks + P->n_cols);
+    t.n_solo = (int32_t)P->n_t_solo;
     t.meta = P->d_t_meta;
     t.ent = P->d_t_ent;
-    t.n_chunks = (int32_t)P->n_t_chunks;
-    t.chunk_beg = P->d_t_chunk_beg;
-    t.chunk_end = P->d_t_chunk_end;
     t.chunk_flag = P->d_t_chunk_flag;
     t.claims = P->d_claims;
     t.mult = P->d_mult;

@@ -104,9 +104,8 @@ struct cbm_plan {
   int64_t* d_t_ptr = nullptr;
   uint32_t* d_t_ent = nullptr;     // row (or slot) | internal << 30 | sign << 31
   int64_t n_t_chunks = 0;
+  int64_t n_t_solo = 0;            // the first of its records: lists a warp takes alone
   int4* d_t_meta = nullptr;        // one record per column, longest lists first (TrArgs)
-  int64_t* d_t_chunk_beg = nullptr;
-  int64_t* d_t_chunk_end = nullptr;
   unsigned* d_t_chunk_flag = nullptr;
 
   std::vector<void*> bufs, chunk_bufs, adj_bufs, adj_chunk_bufs;
