@@ -172,6 +172,14 @@ static __device__ __noinline__ bool wait_flag(const unsigned int* flag, unsigned
   return false;
 }
 
+// One round of a wait that polls several flags: sleeps, and says whether the
+// time is over (or an earlier wait of the launch has failed).  t0: 0 at first.
+static __device__ __noinline__ bool poll_over(unsigned long long& t0, QueueState* qs, long long timeout_ns) {
+  if (t0 == 0) t0 = global_ns();
+  __nanosleep(64);
+  return *(volatile int*)&qs->error != 0 || (long long)(global_ns() - t0) > timeout_ns;
+}
+
 // ---- vector loads / stores ---------------------------------------------------
 template <typename T, int V>
 struct Vec;
@@ -363,19 +371,32 @@ struct Raw<__nv_bfloat16, 1> {
   }
 };
 
+// How the register kernel claims and gathers (CLAIMS).  With two groups claimed
+// ahead, the first third of the resident warps takes all the rows of a plan that has
+// one group of them per warp, longest rows first, and works through them with the
+// rest of the chip idle; and on such a plan the time is the chain of gathers of the
+// longest rows, so more of them in flight count for more than occupancy.  Small
+// plans (the rule is at the launch) therefore claim one group at a time; teams of 8
+// lanes and more also keep twice the gathers in flight (narrower ones gather no
+// faster so: 8,000 nodes, 24 BF16 columns 65 -> 72 us).  Measured on B200, two groups
+// ahead -> as here (us, bit-identical): 8,000 nodes of mean degree 30, shallow tree, 128
+// FP32 / 256 BF16 columns 66 / 87 -> 38 / 42; 2,000 nodes, GIN with 128 / 256 columns 60 /
+// 74 -> 27 / 40; GCN graph of 20,000 nodes, 128 / 256 columns 56 / 65 -> 44 / 48; 4,096
+// nodes, 64 columns 14.6 -> 11.9.  Twice the gathers on large plans cost a resident
+// block and were slower (170,000-node GCN graph, 128 BF16 columns: 152 -> 174).
+enum RowClaims : int {
+  CLAIMS_AHEAD = 0,  // the next two groups claimed while one is worked on
+  CLAIMS_LONE = 1,   // one group at a time
+  CLAIMS_FEW = 2     // one group at a time, twice the gathers in flight
+};
+
 // Gathers in flight per lane: 16 registers' worth (32 from four pieces per lane
-// on), at most 8.  Twice as many cost a resident block and were slower (GCN
-// graph, 128 BF16 columns: 152 -> 174 us, 64-column GIN 81 -> 90).
-template <typename XT, int VPL, int V>
+// on and with CLAIMS_FEW), at most 8.
+template <typename XT, int VPL, int V, int CLAIMS>
 __host__ __device__ constexpr int reg_in_flight() {
-  const int u = (VPL >= 4 ? 32 : 16) / (VPL * Raw<XT, V>::regs);
+  const int u = (VPL >= 4 || CLAIMS == CLAIMS_FEW ? 32 : 16) / (VPL * Raw<XT, V>::regs);
   return u < 1 ? 1 : (u > 8 ? 8 : u);
 }
-// The same where a plan has so few rows that a warp gets one group of them at
-// most (FORM_FEW): occupancy then buys nothing, and a row of 30 entries is four
-// exposed round trips instead of eight (4,096 nodes, 64 FP32 columns: 16.5 -> 12.2 us on
-// the device; 128 BF16 columns 23.9 -> 17.8, 4,000 nodes and 47 columns 47 -> 38).
-constexpr int kFewInFlight = 8;
 
 // Entry idx's scale before the row factor: s, the stored value, or s * m[col]
 // (from the plan's array when it has one).
@@ -562,9 +583,9 @@ __device__ __forceinline__ void gather_row(float (&acc)[VPL][V], const Lane<XT, 
 // with four), three where teams share a warp (40 BF16 columns on the GCN
 // graph: 103 against 121) and for two vectors per lane (47 scalar columns: 103
 // against 137 with two).
-template <typename XT, typename YT, int VPL, int FORM, int TLC>
+template <typename XT, typename YT, int VPL, int FORM, int TLC, int CLAIMS>
 __host__ __device__ constexpr int fwd_min_blocks() {
-  return FORM == 2 || VPL > 4 ? 1 : FORM == 3 ? 2 : VPL == 4 ? 2 : VPL == 1 && TLC == 32 ? 4 : 3;
+  return FORM == 2 || VPL > 4 ? 1 : CLAIMS == CLAIMS_FEW || VPL == 4 ? 2 : VPL == 1 && TLC == 32 ? 4 : 3;
 }
 
 // s + e == a + b exactly (Knuth's TwoSum; explicit roundings, no contraction)
@@ -614,7 +635,9 @@ __device__ __forceinline__ void finish_block(QueueState* qs, unsigned epoch, boo
 // wait then holds up the whole warp, which is safe as long as what it waits
 // for is not the warp's own: an item whose parent lies fewer than 32 queue
 // positions before it carries kNearBit, and a group of items with one runs its
-// row ends team by team, in queue order.
+// row ends team by team, in queue order; with one group claimed at a time (small
+// plans, whose levels may be narrower than a warp) all teams at once whose parents
+// are ready, polled without blocking (2,145 nodes, 16 BF16 columns: 39 us one by one).
 //
 // Progress: a warp finishes its groups in the order it claimed them, also with
 // the next claim already made, and an item depends on earlier items only.
@@ -641,15 +664,16 @@ static_assert(chunk_stop(INT_MAX, kPreMark) == INT_MAX && chunk_stop(5, 12) == 5
               "a presummed row's record, whose mark has no negative, walks no chunks");
 
 // What a register-kernel instantiation leaves out: FORM_PLAIN has no GIN term
-// and no compensation, nor has FORM_FEW, which keeps more gathers in flight.
-enum RowForm : int { FORM_PLAIN = 0, FORM_GIN = 1, FORM_COMP = 2, FORM_FEW = 3 };
+// and no compensation.
+enum RowForm : int { FORM_PLAIN = 0, FORM_GIN = 1, FORM_COMP = 2 };
 
-template <typename XT, typename YT, int VPL, int V, int FORM, int TLC>
-__global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, TLC>())) fwd_kernel(const FwdArgs a) {
+template <typename XT, typename YT, int VPL, int V, int FORM, int TLC, int CLAIMS>
+__global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, TLC, CLAIMS>())) fwd_kernel(const FwdArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr bool COMP = FORM == FORM_COMP;
-  constexpr bool kPlain = FORM == FORM_PLAIN || FORM == FORM_FEW;
-  constexpr int U = FORM == FORM_FEW ? kFewInFlight : reg_in_flight<XT, VPL, V>();
+  constexpr bool kPlain = FORM == FORM_PLAIN;
+  constexpr bool AHEAD = CLAIMS == CLAIMS_AHEAD;
+  constexpr int U = reg_in_flight<XT, VPL, V, CLAIMS>();
   // parents' rows come from the FP32 state rows
   const bool state = sizeof(YT) != 4 || FORM == FORM_GIN || (COMP && a.gin);
   const int lane = threadIdx.x & 31;
@@ -730,239 +754,270 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
   }
 
   // ---- rows: one group of `teams` items per claim from the warp's queue, the
-  // next claim made ahead
+  // next claim made ahead if AHEAD
   const unsigned wq = threadIdx.x >> 5;
   unsigned pend = 0;
-  if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+  auto claim = [&] {
+    if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+  };
   // first item of the warp's next group; n when the queue is exhausted
   auto next_group = [&]() -> unsigned {
     const unsigned g = (__shfl_sync(kAll, pend, 0) * kClaimQueues + wq) * teams;
     if (g >= n) return n;  // the claim stays pending: every later call ends here too
-    if (lane == 0) pend = atomicAdd(a.claims + wq * kClaimStride, 1u);
+    if (AHEAD) claim();
     return g;
   };
-  unsigned g0 = next_group();
-  if (g0 < n) {
-    int4 m0 = __ldg(a.meta + g0 + team);
-    uint32_t e0 = 0;
-    float s0 = 0.f;
-    unsigned f0 = 0;
+  unsigned g0, g1 = n, f0;
+  int4 m0, m1;
+  uint32_t e0;
+  float s0;
+  // the next group, with nothing of it claimed or loaded yet
+  auto begin = [&] {
+    claim();
+    g0 = next_group();
+    if (g0 >= n) return;
+    m0 = __ldg(a.meta + g0 + team);
+    e0 = 0;
+    s0 = 0.f;
+    f0 = 0;
     if (tl < m0.w) {
       e0 = __ldg(a.ent + (uint32_t)m0.z + tl);
       s0 = reg_scale(e0, vals ? vals + (uint32_t)m0.z : nullptr, tl, a.scale_mode, a.mult);
     }
-    unsigned g1 = next_group();
-    int4 m1 = __ldg(a.meta + g1 + team);
+    if (AHEAD) g1 = next_group();
+    m1 = __ldg(a.meta + g1 + team);
     if (a.skip_parent) m0.y = -1, m1.y = -1;
     if (m0.y >= 0) f0 = ld_acquire(a.node_flag + m0.y);
-    while (g0 < n) {
-      const unsigned item = g0 + team;
-      const bool have = TLC == 32 || item < n;
-      const int node = m0.x & kNodeMask;
-      const int p = m0.y;
-      const float dv = drow || ratio ? __ldg(a.mult + node) : 1.f;
-      // the parent's row, if that is final already
-      const bool ready = p >= 0 && f0 == epoch;
-      float yp[VPL][V];
-      float dp = 1.f;
-      auto load_parent = [&]() {
-        const float* src;
-        if (state) {
-          src = a.pstate + (int64_t)__ldg(a.rec_par_slot + item) * a.ldp;
-        } else {
-          src = static_cast<const float*>(a.y) + row_off(p, a.ldy);
-        }
+  };
+  begin();
+  while (g0 < n) {
+    const unsigned item = g0 + team;
+    const bool have = TLC == 32 || item < n;
+    const int node = m0.x & kNodeMask;
+    const int p = m0.y;
+    const float dv = drow || ratio ? __ldg(a.mult + node) : 1.f;
+    // the parent's row, if that is final already
+    const bool ready = p >= 0 && f0 == epoch;
+    float yp[VPL][V];
+    float dp = 1.f;
+    auto load_parent = [&]() {
+      const float* src;
+      if (state) {
+        src = a.pstate + (int64_t)__ldg(a.rec_par_slot + item) * a.ldp;
+      } else {
+        src = static_cast<const float*>(a.y) + row_off(p, a.ldy);
+      }
 #pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          const int vi = tl + v * TL;
-          if (vi < a.nvec) load_f32_cg<V>(src + (int64_t)vi * V, yp[v]);
-        }
-      };
-      if (ready) load_parent();
-      typename Raw<XT, V>::type xself[VPL];  // GIN: the row's own X, for its store
-      auto load_self = [&]() {
+      for (int v = 0; v < VPL; ++v) {
+        const int vi = tl + v * TL;
+        if (vi < a.nvec) load_f32_cg<V>(src + (int64_t)vi * V, yp[v]);
+      }
+    };
+    if (ready) load_parent();
+    typename Raw<XT, V>::type xself[VPL];  // GIN: the row's own X, for its store
+    auto load_self = [&]() {
 #pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-          xself[v] = Raw<XT, V>::zero();
-          if (a.gin && have) xself[v] = Raw<XT, V>::load(reinterpret_cast<const XT*>(ln.row(node) + ln.off[v]));
-        }
-      };
-      // ahead of the gathers, but for one piece per lane, where those registers
-      // are worth more as occupancy (100,000-node GIN, 256 FP32 columns: 198 ->
-      // 178 us; 200,000 nodes, 128 columns: 376 -> 353 us the other way)
-      if (!kPlain && VPL > 1) load_self();
-      if (ratio && p >= 0) dp = __ldg(a.mult + p);
-      float acc[VPL][V];
+      for (int v = 0; v < VPL; ++v) {
+        xself[v] = Raw<XT, V>::zero();
+        if (a.gin && have) xself[v] = Raw<XT, V>::load(reinterpret_cast<const XT*>(ln.row(node) + ln.off[v]));
+      }
+    };
+    // ahead of the gathers, but for one piece per lane, where those registers
+    // are worth more as occupancy (100,000-node GIN, 256 FP32 columns: 198 ->
+    // 178 us; 200,000 nodes, 128 columns: 376 -> 353 us the other way)
+    if (!kPlain && VPL > 1) load_self();
+    if (ratio && p >= 0) dp = __ldg(a.mult + p);
+    float acc[VPL][V];
 #pragma unroll
-      for (int v = 0; v < VPL; ++v)
+    for (int v = 0; v < VPL; ++v)
 #pragma unroll
-        for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
-      const int len = m0.w > 0 ? m0.w : 0;
-      uint32_t e1 = 0;
-      float s1 = 0.f;
-      unsigned f1 = 0;
-      gather_row<XT, VPL, V, TLC, U>(acc, ln, a.ent + (uint32_t)m0.z, vals ? vals + (uint32_t)m0.z : nullptr, len,
-                                  TLC == 32 ? len : __reduce_max_sync(kAll, len), e0, s0, drow ? dv : 1.f,
-                                  a.scale_mode, a.mult, tl, TL, [&] {
-                                    if (tl < m1.w) {
-                                      e1 = __ldg(a.ent + (uint32_t)m1.z + tl);
-                                      if (vals) s1 = __ldg(vals + (uint32_t)m1.z + tl);
-                                    }
-                                    if (m1.y >= 0) f1 = ld_acquire(a.node_flag + m1.y);
-                                  });
+      for (int q = 0; q < V; ++q) acc[v][q] = 0.f;
+    const int len = m0.w > 0 ? m0.w : 0;
+    uint32_t e1 = 0;
+    float s1 = 0.f;
+    unsigned f1 = 0;
+    gather_row<XT, VPL, V, TLC, U>(acc, ln, a.ent + (uint32_t)m0.z, vals ? vals + (uint32_t)m0.z : nullptr, len,
+                                TLC == 32 ? len : __reduce_max_sync(kAll, len), e0, s0, drow ? dv : 1.f,
+                                a.scale_mode, a.mult, tl, TL, [&] {
+                                  if (tl < m1.w) {
+                                    e1 = __ldg(a.ent + (uint32_t)m1.z + tl);
+                                    if (vals) s1 = __ldg(vals + (uint32_t)m1.z + tl);
+                                  }
+                                  if (m1.y >= 0) f1 = ld_acquire(a.node_flag + m1.y);
+                                });
 
-      if (!kPlain && VPL == 1) load_self();
+    if (!kPlain && VPL == 1) load_self();
 
-      // ---- the row's end: chunk partials, parent, store, ready flag
-      const int serial = TLC != 32 && __any_sync(kAll, have && (m0.x & kNearBit) != 0) ? (int)teams : 1;
-      for (int t = 0; t < serial; ++t) {
-        if (have && (serial == 1 || team == t)) {
-          if (m0.w == kPreMark) {
-            // summed ahead: record z is its place among the presummed rows
-            if (wait_flag(a.chunk_flag + n_split + m0.z, epoch, a.qs, a.timeout_ns, (long long)m0.z)) {
-              const float* prow = a.pre_rows ? a.pre_rows + (int64_t)m0.z * a.ldp
-                                             : static_cast<const float*>(a.y) + row_off(node, a.ldy);
-#pragma unroll
-              for (int v = 0; v < VPL; ++v) {
-                const int vi = tl + v * TL;
-                if (vi < a.nvec) load_f32_cg<V>(prow + vi * V, acc[v]);
-              }
-            }
-          }
-          for (int k = m0.z, ke = chunk_stop(m0.z, m0.w); k < ke; ++k) {
-            if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
-            const float* prow = a.partial + (int64_t)k * a.ldp;
+    // ---- the row's end: chunk partials, parent, store, ready flag
+    const bool near_any = TLC != 32 && __any_sync(kAll, have && (m0.x & kNearBit) != 0);
+    bool todo = have, more = false;
+    int turn = 0;
+    unsigned long long t0 = 0;
+    do {
+      bool go = todo;
+      if constexpr (AHEAD) {
+        // a group that may hold an item and its parent: team by team, in queue order
+        go = have && (!near_any || team == turn);
+        more = near_any && ++turn < (int)teams;
+      } else if (near_any) {
+        // here those whose parent is ready
+        if (go && p >= 0) go = ld_acquire(a.node_flag + p) == epoch;
+        go = __shfl_sync(kAll, go, team * TL);  // the team's first lane's answer
+        if (!__any_sync(kAll, go)) go = todo && poll_over(t0, a.qs, a.timeout_ns);
+        go = __shfl_sync(kAll, go, team * TL);
+      }
+      if (go) {
+        todo = false;
+        if (m0.w == kPreMark) {
+          // summed ahead: record z is its place among the presummed rows
+          if (wait_flag(a.chunk_flag + n_split + m0.z, epoch, a.qs, a.timeout_ns, (long long)m0.z)) {
+            const float* prow = a.pre_rows ? a.pre_rows + (int64_t)m0.z * a.ldp
+                                           : static_cast<const float*>(a.y) + row_off(node, a.ldy);
 #pragma unroll
             for (int v = 0; v < VPL; ++v) {
               const int vi = tl + v * TL;
-              if (vi < a.nvec) {
-                float part[V];
-                load_f32_cg<V>(prow + vi * V, part);
-#pragma unroll
-                for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], part[q]);
-              }
+              if (vi < a.nvec) load_f32_cg<V>(prow + vi * V, acc[v]);
             }
           }
-          // compensated arithmetic for this row, a residual to read from the parent
-          const bool cmode = COMP && (int)item >= a.comp_item0;
-          const bool cread = COMP && (int)item >= a.comp_read0;
-          float cres[VPL][V];  // unused (and removed by the compiler) without COMP
-#pragma unroll
-          for (int v = 0; v < VPL; ++v)
-#pragma unroll
-            for (int q = 0; q < V; ++q) cres[v][q] = 0.f;
-          // after a failed (timed-out) wait the parent is left out; the error is recorded
-          bool add = ready;
-          if (p >= 0 && !ready && wait_flag(a.node_flag + p, epoch, a.qs, a.timeout_ns, (long long)node)) {
-            load_parent();
-            add = true;
-          }
-          if (add) {
-#pragma unroll
-            for (int v = 0; v < VPL; ++v) {
-              const int vi = tl + v * TL;
-              if (vi < a.nvec) {
-                if (COMP && cmode) {
-                  // parent value = yp + rp (rp: its residual); add with TwoSum and keep
-                  // the rounding errors (of the ratio's product and quotient too)
-                  float rp[V];
-                  if (cread) {
-                    load_f32_cg<V>(a.pcomp + (int64_t)__ldg(a.rec_par_slot + item) * a.ldp + vi * V, rp);
-                  } else {
-#pragma unroll
-                    for (int q = 0; q < V; ++q) rp[q] = 0.f;
-                  }
-#pragma unroll
-                  for (int q = 0; q < V; ++q) {
-                    float y = yp[v][q], r = rp[q];
-                    if (ratio) {
-                      const float prod = __fmul_rn(yp[v][q], dv);
-                      const float pe = fmaf(yp[v][q], dv, -prod);  // prod + pe == yp * dv
-                      y = __fdiv_rn(prod, dp);
-                      const float qe = __fdiv_rn(fmaf(-y, dp, prod), dp);  // y + qe ~ prod / dp
-                      r = __fadd_rn(__fdiv_rn(fmaf(r, dv, pe), dp), qe);
-                    }
-                    float s_, e_;
-                    two_sum(acc[v][q], y, s_, e_);
-                    acc[v][q] = s_;
-                    cres[v][q] = __fadd_rn(r, e_);
-                  }
-                } else if (ratio) {
-#pragma unroll
-                  for (int q = 0; q < V; ++q)
-                    acc[v][q] = __fadd_rn(acc[v][q], __fdiv_rn(__fmul_rn(yp[v][q], dv), dp));
-                } else {
-#pragma unroll
-                  for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], yp[v][q]);
-                }
-              }
-            }
-          }
-          const bool keep = m0.x < 0 && !a.skip_parent;  // children read this row
-          const int ss = keep && (state || COMP) ? __ldg(a.rec_self_slot + item) : 0;
-          if (COMP && cmode) {
-            // the row's value is acc + cres, rounded once; its residual is kept for
-            // the children of an internal node
-#pragma unroll
-            for (int v = 0; v < VPL; ++v)
-#pragma unroll
-              for (int q = 0; q < V; ++q) {
-                float s_, e_;
-                two_sum(acc[v][q], cres[v][q], s_, e_);
-                acc[v][q] = s_;
-                cres[v][q] = e_;
-              }
-            if (keep) {
-              float* crow = a.pcomp + (int64_t)ss * a.ldp;
-#pragma unroll
-              for (int v = 0; v < VPL; ++v) {
-                const int vi = tl + v * TL;
-                if (vi < a.nvec) store_f32<V>(crow + vi * V, cres[v]);
-              }
-            }
-          }
-          YT* yrow = static_cast<YT*>(a.y) + row_off(node, a.ldy);
+        }
+        for (int k = m0.z, ke = chunk_stop(m0.z, m0.w); k < ke; ++k) {
+          if (!wait_flag(a.chunk_flag + k, epoch, a.qs, a.timeout_ns, (long long)k)) continue;
+          const float* prow = a.partial + (int64_t)k * a.ldp;
 #pragma unroll
           for (int v = 0; v < VPL; ++v) {
             const int vi = tl + v * TL;
             if (vi < a.nvec) {
-              if constexpr (kPlain) {
-                store_vec<YT, V>(yrow + (int64_t)vi * V, acc[v]);
-              } else {
-                float xs[V], out[V];
-                Raw<XT, V>::widen(xself[v], xs);
+              float part[V];
+              load_f32_cg<V>(prow + vi * V, part);
 #pragma unroll
-                for (int q = 0; q < V; ++q) out[q] = a.gin ? fmaf(a.gin_scale, xs[q], acc[v][q]) : acc[v][q];
-                store_vec<YT, V>(yrow + (int64_t)vi * V, out);
-              }
+              for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], part[q]);
             }
-          }
-          if (keep) {
-            if (state) {
-              float* srow = a.pstate + (int64_t)ss * a.ldp;
-#pragma unroll
-              for (int v = 0; v < VPL; ++v) {
-                const int vi = tl + v * TL;
-                if (vi < a.nvec) store_f32<V>(srow + vi * V, acc[v]);
-              }
-            }
-            // as for the chunks: the team's stores before its first lane's release
-            __syncwarp(TLC == 32 || TL == 32 ? kAll : (((1u << TL) - 1u) << (team * TL)));
-            if (tl == 0) st_release(a.node_flag + node, epoch);
           }
         }
-        __syncwarp();
+        // compensated arithmetic for this row, a residual to read from the parent
+        const bool cmode = COMP && (int)item >= a.comp_item0;
+        const bool cread = COMP && (int)item >= a.comp_read0;
+        float cres[VPL][V];  // unused (and removed by the compiler) without COMP
+#pragma unroll
+        for (int v = 0; v < VPL; ++v)
+#pragma unroll
+          for (int q = 0; q < V; ++q) cres[v][q] = 0.f;
+        // after a failed (timed-out) wait the parent is left out; the error is recorded
+        bool add = ready;
+        if (p >= 0 && !ready && wait_flag(a.node_flag + p, epoch, a.qs, a.timeout_ns, (long long)node)) {
+          load_parent();
+          add = true;
+        }
+        if (add) {
+#pragma unroll
+          for (int v = 0; v < VPL; ++v) {
+            const int vi = tl + v * TL;
+            if (vi < a.nvec) {
+              if (COMP && cmode) {
+                // parent value = yp + rp (rp: its residual); add with TwoSum and keep
+                // the rounding errors (of the ratio's product and quotient too)
+                float rp[V];
+                if (cread) {
+                  load_f32_cg<V>(a.pcomp + (int64_t)__ldg(a.rec_par_slot + item) * a.ldp + vi * V, rp);
+                } else {
+#pragma unroll
+                  for (int q = 0; q < V; ++q) rp[q] = 0.f;
+                }
+#pragma unroll
+                for (int q = 0; q < V; ++q) {
+                  float y = yp[v][q], r = rp[q];
+                  if (ratio) {
+                    const float prod = __fmul_rn(yp[v][q], dv);
+                    const float pe = fmaf(yp[v][q], dv, -prod);  // prod + pe == yp * dv
+                    y = __fdiv_rn(prod, dp);
+                    const float qe = __fdiv_rn(fmaf(-y, dp, prod), dp);  // y + qe ~ prod / dp
+                    r = __fadd_rn(__fdiv_rn(fmaf(r, dv, pe), dp), qe);
+                  }
+                  float s_, e_;
+                  two_sum(acc[v][q], y, s_, e_);
+                  acc[v][q] = s_;
+                  cres[v][q] = __fadd_rn(r, e_);
+                }
+              } else if (ratio) {
+#pragma unroll
+                for (int q = 0; q < V; ++q)
+                  acc[v][q] = __fadd_rn(acc[v][q], __fdiv_rn(__fmul_rn(yp[v][q], dv), dp));
+              } else {
+#pragma unroll
+                for (int q = 0; q < V; ++q) acc[v][q] = __fadd_rn(acc[v][q], yp[v][q]);
+              }
+            }
+          }
+        }
+        const bool keep = m0.x < 0 && !a.skip_parent;  // children read this row
+        const int ss = keep && (state || COMP) ? __ldg(a.rec_self_slot + item) : 0;
+        if (COMP && cmode) {
+          // the row's value is acc + cres, rounded once; its residual is kept for
+          // the children of an internal node
+#pragma unroll
+          for (int v = 0; v < VPL; ++v)
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+              float s_, e_;
+              two_sum(acc[v][q], cres[v][q], s_, e_);
+              acc[v][q] = s_;
+              cres[v][q] = e_;
+            }
+          if (keep) {
+            float* crow = a.pcomp + (int64_t)ss * a.ldp;
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) {
+              const int vi = tl + v * TL;
+              if (vi < a.nvec) store_f32<V>(crow + vi * V, cres[v]);
+            }
+          }
+        }
+        YT* yrow = static_cast<YT*>(a.y) + row_off(node, a.ldy);
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          const int vi = tl + v * TL;
+          if (vi < a.nvec) {
+            if constexpr (kPlain) {
+              store_vec<YT, V>(yrow + (int64_t)vi * V, acc[v]);
+            } else {
+              float xs[V], out[V];
+              Raw<XT, V>::widen(xself[v], xs);
+#pragma unroll
+              for (int q = 0; q < V; ++q) out[q] = a.gin ? fmaf(a.gin_scale, xs[q], acc[v][q]) : acc[v][q];
+              store_vec<YT, V>(yrow + (int64_t)vi * V, out);
+            }
+          }
+        }
+        if (keep) {
+          if (state) {
+            float* srow = a.pstate + (int64_t)ss * a.ldp;
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) {
+              const int vi = tl + v * TL;
+              if (vi < a.nvec) store_f32<V>(srow + vi * V, acc[v]);
+            }
+          }
+          // as for the chunks: the team's stores before its first lane's release
+          __syncwarp(TLC == 32 || TL == 32 ? kAll : (((1u << TL) - 1u) << (team * TL)));
+          if (tl == 0) st_release(a.node_flag + node, epoch);
+        }
       }
-      // ---- on to the next row: its entries are here, the record behind it loads
-      g0 = g1;
-      m0 = m1;
-      e0 = e1;
-      s0 = vals ? s1 : tl < m0.w ? reg_scale(e0, nullptr, 0, a.scale_mode, a.mult) : 0.f;
-      f0 = f1;
-      g1 = next_group();
-      m1 = __ldg(a.meta + g1 + team);
-      if (a.skip_parent) m1.y = -1;
+      __syncwarp();
+      if constexpr (!AHEAD) more = near_any && __any_sync(kAll, todo);
+    } while (more);
+    // ---- on to the next row: its entries are here, the record behind it loads
+    if constexpr (!AHEAD) {
+      begin();
+      continue;
     }
+    g0 = g1;
+    m0 = m1;
+    e0 = e1;
+    s0 = vals ? s1 : tl < m0.w ? reg_scale(e0, nullptr, 0, a.scale_mode, a.mult) : 0.f;
+    f0 = f1;
+    g1 = next_group();
+    m1 = __ldg(a.meta + g1 + team);
+    if (a.skip_parent) m1.y = -1;
   }
   finish_block(a.qs, epoch, a.publish_epoch != 0, a.claims);
 }

@@ -43,17 +43,20 @@ int cached_grid(GridCache& c, K kernel, int device, int block, int smem) {
   return g;
 }
 
-template <typename XT, typename YT, int VPL, int V, int FORM>
-int launch_fwd_t(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
+template <typename XT, typename YT, int VPL, int V, int FORM, int CLAIMS>
+int launch_fwd_claims(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
   // full-warp teams have their own instantiation (also where X's rows lie 2^32
   // bytes apart or more: that one has 32-bit row strides)
   static GridCache cache[3];
   int form = a.team == 32 && (uint64_t)a.ldx * sizeof(XT) <= 0xffffffffull ? 1 : 0;
-  auto kern = form == 1 ? fwd_kernel<XT, YT, VPL, V, FORM, 32> : fwd_kernel<XT, YT, VPL, V, FORM, kTeamAny>;
-  if constexpr (VPL == 1 && FORM != FORM_FEW) {
+  auto kern = fwd_kernel<XT, YT, VPL, V, FORM, kTeamAny, CLAIMS>;
+  if constexpr (CLAIMS != CLAIMS_LONE) {
+    if (form == 1) kern = fwd_kernel<XT, YT, VPL, V, FORM, 32, CLAIMS>;
+  }
+  if constexpr (VPL == 1 && CLAIMS != CLAIMS_FEW) {
     if (a.team <= 2) {
       form = 2;
-      kern = fwd_kernel<XT, YT, VPL, V, FORM, kTeamNarrow>;
+      kern = fwd_kernel<XT, YT, VPL, V, FORM, kTeamNarrow, CLAIMS>;
     }
   }
   const int grid = cached_grid(cache[form], kern, P->device, kThreads, 0);
@@ -62,6 +65,22 @@ int launch_fwd_t(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
   P->launches++;
   P->last_grid = grid;
   return cuda_status(cudaGetLastError());
+}
+
+template <typename XT, typename YT, int VPL, int V, int FORM>
+int launch_fwd_t(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
+  // Small plans: at most 8 groups for each warp of three blocks per SM (28,416 groups on
+  // B200).  With the line at one group or at three, the cases above it keep the
+  // times of claims ahead (RowClaims): 8,000 rows of 128 columns 66-71 us, 38 below it;
+  // 20,000 rows 72-75 against 59.  At 16, GIN on 100,000 rows of 64 columns: 78 -> 84 us.
+  if constexpr (VPL <= 2 && FORM != FORM_COMP) {
+    const int64_t groups = ((int64_t)a.n_items * a.team + 31) / 32;
+    if (groups <= (int64_t)sm_count(P->device) * 24 * 8) {
+      if (a.team >= 8) return launch_fwd_claims<XT, YT, VPL, V, FORM, CLAIMS_FEW>(P, a, st);
+      if constexpr (VPL == 1) return launch_fwd_claims<XT, YT, VPL, V, FORM, CLAIMS_LONE>(P, a, st);
+    }
+  }
+  return launch_fwd_claims<XT, YT, VPL, V, FORM, CLAIMS_AHEAD>(P, a, st);
 }
 
 template <typename XT, typename YT, int TL, int VPL, int V, int S, bool TMA = false>
@@ -139,13 +158,6 @@ int launch_tma_any(cbm_plan* P, const FwdArgs& a, int team, int vpl, const CUten
 
 template <typename XT, typename YT, int V, int FORM>
 int launch_fwd_v(cbm_plan* P, const FwdArgs& a, int vpl, cudaStream_t st) {
-  // few rows: one group per warp at 16 resident warps per SM (narrower teams are
-  // slower so: 8,000 nodes, 24 BF16 columns 64 -> 71 us)
-  if constexpr (FORM == FORM_PLAIN) {
-    const int64_t groups = ((int64_t)a.n_items * a.team + 31) / 32;
-    if (vpl == 1 && a.team >= 8 && groups <= (int64_t)sm_count(P->device) * 16)
-      return launch_fwd_t<XT, YT, 1, V, FORM_FEW>(P, a, st);
-  }
   switch (vpl) {
     case 1: return launch_fwd_t<XT, YT, 1, V, FORM>(P, a, st);
     case 2: return launch_fwd_t<XT, YT, 2, V, FORM>(P, a, st);
