@@ -18,7 +18,8 @@ on the GPU through the library's stateless ``cbm_s_*`` entry points
 (include/cbm_b200.h), straight from the arguments' CSR arrays and tree edges:
 
 * CUDA tensors (all on one device): the call is queued on the current stream
-  and returns at once, like any CUDA operator; device-side errors (an index
+  and returns at once, like any CUDA operator (products on several streams
+  have a workspace each); device-side errors (an index
   out of range, a node with two parents, a child edge listed before its
   parent's) are recorded and raised by ``check_device()``.
 * CPU tensors (the reference's own convention): the operands are copied to the
@@ -35,6 +36,7 @@ products raise RuntimeError.
 from __future__ import annotations
 
 import ctypes as C
+import threading
 from dataclasses import dataclass
 
 import numpy as np
@@ -214,36 +216,77 @@ def build_cached(row, col, n_rows, alpha=0, cache_dir=None, n_threads=0, cluster
 
 # ---- the reference's CPU products, on the GPU ------------------------------------
 
-_WORKSPACE = {}  # device index -> zero-filled uint8 tensor (status word + per-node stamps)
+# Workspaces (zero-filled uint8: status word, claim counters, per-node stamps), by
+# (device index, stream handle): a product owns its workspace while it runs, and
+# products on several streams run at once.  Each is allocated with its stream
+# current, so that the allocator gives it back in that stream's order.  At most
+# _MAX_STREAMS of a device are kept, the least recently used go first; the
+# status of one that goes is carried over in _CARRIED.  A workspace that a captured
+# graph holds stays, under (device index, (address,)).
+_MAX_STREAMS = 32
+_WORKSPACE = {}
+_CARRIED = {}
+_LOCK = threading.Lock()
 
 
-def _workspace(device, rows):
-    """The device's workspace, grown to ``rows`` nodes (its status word carried over)."""
-    lib = _lib.load()
-    need = max(int(lib.cbm_direct_workspace_bytes(int(rows))), 256)
-    ws = _WORKSPACE.get(device.index)
-    if ws is None or ws.numel() < need:
-        grown = torch.zeros(max(need, 2 * ws.numel() if ws is not None else 0), dtype=torch.uint8, device=device)
-        if ws is not None:
-            grown[:256].copy_(ws[:256])
-        _WORKSPACE[device.index] = ws = grown
+def _capturing():
+    return torch.cuda.is_current_stream_capturing()
+
+
+def _status(ws, stream):
+    st, info = C.c_int32(0), C.c_int64(0)
+    _lib.check(_lib.load().cbm_direct_status(ws.data_ptr(), C.c_void_p(stream), C.byref(st), C.byref(info)),
+               "cbm_direct_status")
+    return int(st.value), int(info.value)
+
+
+def _workspace(device, rows, stream):
+    """The workspace of ``stream`` on ``device``, grown to ``rows`` nodes (its status
+    word carried over)."""
+    need = max(int(_lib.load().cbm_direct_workspace_bytes(int(rows))), 256)
+    key = (device.index, stream)
+    with _LOCK:
+        ws = _WORKSPACE.get(key)
+        held = [k for k in _WORKSPACE if k[0] == device.index and isinstance(k[1], int) and k != key]
+        if _capturing():
+            # the graph takes a workspace that is there: the stream's own, else another
+            # stream's, which products there must then not use while the graph runs;
+            # else a new one, zeroed by the graph
+            fit = [w for w in [ws] + [_WORKSPACE[k] for k in reversed(held)] if w is not None and w.numel() >= need]
+            if fit:
+                _WORKSPACE[(device.index, (fit[0].data_ptr(),))] = fit[0]
+                return fit[0]
+            own = torch.zeros(need, dtype=torch.uint8, device=device)
+            _WORKSPACE[(device.index, (own.data_ptr(),))] = own
+            return own
+        if ws is None or ws.numel() < need:
+            grown = torch.zeros(max(need, 2 * ws.numel() if ws is not None else 0), dtype=torch.uint8, device=device)
+            if ws is not None:
+                grown[:256].copy_(ws[:256])
+            ws = grown
+        if len(held) >= _MAX_STREAMS:
+            torch.cuda.synchronize(device)
+            status = _status(_WORKSPACE.pop(held[0]), stream)
+            if status[0] != _lib.OK:
+                _CARRIED.setdefault(device.index, status)
+        _WORKSPACE.pop(key, None)  # the most recently used is the last
+        _WORKSPACE[key] = ws
     return ws
 
 
 def device_status(device=None):
-    """Synchronises the current stream of ``device`` and returns (status, info):
-    the first device-side error the products recorded since the last query
-    (status 0: none), then clears it."""
+    """Synchronises the current stream of ``device`` (the device, where products ran
+    on several streams) and returns (status, info): the first device-side error
+    the products recorded since the last query (status 0: none), then clears it."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    ws = _WORKSPACE.get(device.index)
-    if ws is None:
-        return _lib.OK, 0
-    st = C.c_int32(0)
-    info = C.c_int64(0)
-    with torch.cuda.device(device):
-        _lib.check(_lib.load().cbm_direct_status(ws.data_ptr(), C.c_void_p(torch.cuda.current_stream().cuda_stream),
-                                                 C.byref(st), C.byref(info)), "cbm_direct_status")
-    return int(st.value), int(info.value)
+    with _LOCK, torch.cuda.device(device):
+        index, stream = torch.cuda.current_device(), torch.cuda.current_stream().cuda_stream
+        used = {k: ws for k, ws in _WORKSPACE.items() if k[0] == index}
+        found = [_CARRIED.pop(index)] if index in _CARRIED else []
+        if set(used) - {(index, stream)}:
+            torch.cuda.synchronize(device)
+        found += [_status(ws, stream) for ws in used.values()]
+    return next((f for f in found if f[0] != _lib.OK), (_lib.OK, 0))
 
 
 def check_device(device=None):
@@ -288,15 +331,15 @@ def _run(entry, named, make_args):
                 raise RuntimeError(f'"{name}" must be contiguous')
         dev = tensors
     with torch.cuda.device(device):
-        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        stream = torch.cuda.current_stream().cuda_stream
         out = dev["dst"]
-        ws = _workspace(device, out.shape[0])
+        ws = _workspace(device, out.shape[0], stream)
 
         def ptr(name):
             t = dev[name]
             return t.data_ptr() if t.numel() else None
 
-        rc = getattr(lib, entry)(*build_args(ptr, stream, ws))
+        rc = getattr(lib, entry)(*build_args(ptr, C.c_void_p(stream), ws))
         _lib.check(rc, entry)
         if host:
             tensors["dst"].copy_(out.cpu())
