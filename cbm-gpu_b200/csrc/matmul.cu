@@ -198,7 +198,9 @@ int rebuild_adjoint_chunks(cbm_plan* P, cudaStream_t st) {
   // its chunks' sums)
   auto entries = [&](int64_t j) { return P->h_t_ptr[j + 1] - P->h_t_ptr[j]; };
   auto cost = [&](int64_t j) { return entries(j) > T ? (int64_t)1 : (entries(j) + 3) / 4; };
-  std::vector<int64_t> start(T / 4 + 3, 0);
+  int64_t most = 0;
+  for (int64_t j = 0; j < P->n_cols; ++j) most = std::max(most, cost(j));
+  std::vector<int64_t> start(most + 2, 0);
   std::vector<int4> meta;
   std::vector<int32_t> chunk0(P->n_cols, -1);
   int64_t n_solo = 0;
