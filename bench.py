@@ -482,8 +482,8 @@ def _time_events(fn, steps, warmup):
     return e0.elapsed_time(e1) / steps
 
 
-BATCH_SPACE = {"chunk_nnz": [128, 256], "rows_per_claim": [2, 4, 8], "variant": ["auto", "register"], "team": [0, 8]}
-PREC_SPACE = {"chunk_nnz": [256, 512], "rows_per_claim": [4, 8, 16], "variant": ["auto", "register", "tma"],
+BATCH_SPACE = {"chunk_nnz": [128, 256], "rows_per_claim": [2, 4, 8], "variant": ["register", "staged"], "team": [0, 8]}
+PREC_SPACE = {"chunk_nnz": [256, 512], "rows_per_claim": [4, 8, 16], "variant": ["register", "staged", "tma"],
               "hot_rows": [0, 65536, 262144]}
 
 
@@ -494,7 +494,7 @@ def batch_form(steps, warmup, space=None):
     over ``space``."""
     from cbm import _lib, synthetic
     from cbm.batch import cbm_batch
-    from cbm.tune import autotune
+    from cbm.tune import autotune, candidates
 
     t0 = time.time()
     graphs = synthetic.batch_graphs(512, seed=4)
@@ -504,7 +504,7 @@ def batch_form(steps, warmup, space=None):
     g = torch.Generator(device="cuda").manual_seed(4)
     x = torch.randn(n, 64, device="cuda", generator=g).to(torch.bfloat16)
     y = torch.empty(n, 64, device="cuda")
-    tuned = autotune(b.plan, "dadx", x, y, space=space or BATCH_SPACE)
+    tuned = autotune(b.plan, "dadx", x, y, space=space or candidates(BATCH_SPACE))
     l0 = b.plan.stat(_lib.P_LAUNCHES)
     b.matmul(x, y)  # kernels one product launches (the replay launches the same)
     launches = b.plan.stat(_lib.P_LAUNCHES) - l0
@@ -566,9 +566,9 @@ def precision_form(steps, warmup, prec_nodes=0, space=None, knobs=None):
     if knobs is not None:
         a.plan.tune(**knobs)
     else:
-        from cbm.tune import autotune
+        from cbm.tune import autotune, candidates
 
-        tuned = autotune(a.plan, "adx", x, y, space=space or PREC_SPACE)
+        tuned = autotune(a.plan, "adx", x, y, space=space or candidates(PREC_SPACE))
     ms = _time_events(lambda: a.matmul(x, y), steps, warmup)
     dinv = dinv_f64(ei, n)
     err = {"product": fp64_sample_error(ei, n, x, y, cs=dinv),

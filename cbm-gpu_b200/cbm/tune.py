@@ -15,16 +15,36 @@ import statistics
 
 import torch
 
-__all__ = ["autotune", "DEFAULT_SPACE"]
+__all__ = ["autotune", "candidates", "DEFAULT_SPACE"]
 
 DEFAULT_SPACE = {
     "chunk_nnz": [128, 256, 512],
     "rows_per_claim": [2, 4, 8],
-    "variant": ["auto", "register"],
+    "variant": ["register", "staged"],
     "hot_rows": [0, 65536],
 }
 
+# what the register kernel does not read: it claims one group of rows at a time or
+# two ahead by itself, has its own team sizes and no L2 hints
+_STAGED_ONLY = ("rows_per_claim", "rows_per_claim_deep", "hot_rows", "team")
+
 _cache = {}
+
+
+def _product(space):
+    return [dict(zip(space, values)) for values in itertools.product(*space.values())]
+
+
+def candidates(space):
+    """The configurations of a space, those of the register kernel without the knobs
+    that it does not read (they keep the first value listed)."""
+    out = []
+    for cfg in _product(space):
+        if cfg.get("variant") == "register":
+            cfg.update({k: space[k][0] for k in _STAGED_ONLY if k in cfg})
+        if cfg not in out:
+            out.append(cfg)
+    return out
 
 
 def _time(fn, reps, iters):
@@ -41,17 +61,17 @@ def _time(fn, reps, iters):
 
 
 def autotune(plan, op, x, y, space=None, reps=3, iters=5, warmup=2):
-    """Tunes ``plan`` for y <- op(A) x; returns [(config, ms)] sorted by time."""
+    """Tunes ``plan`` for y <- op(A) x; returns [(config, ms)] sorted by time.
+    ``space``: the values to try of each knob, all combinations of them, or a list of
+    configurations (default: the ``candidates`` of DEFAULT_SPACE)."""
     key = (id(plan), op, x.shape[1], x.dtype, y.dtype)
     if key in _cache:
         best = _cache[key][0][0]
         plan.tune(**best)
         return _cache[key]
-    space = dict(DEFAULT_SPACE if space is None else space)
-    names = list(space)
+    space = candidates(DEFAULT_SPACE) if space is None else _product(space) if isinstance(space, dict) else space
     results = []
-    for values in itertools.product(*(space[k] for k in names)):
-        cfg = dict(zip(names, values))
+    for cfg in space:
         plan.tune(**cfg)
         fn = lambda: plan.matmul(op, x, y)  # noqa: E731
         for _ in range(warmup):
