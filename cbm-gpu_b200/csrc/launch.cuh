@@ -43,6 +43,14 @@ int cached_grid(GridCache& c, K kernel, int device, int block, int smem) {
   return g;
 }
 
+// Small plans: at most 8 groups for each warp of three blocks per SM (28,416 groups on
+// B200).  With the line at one group or at three, the cases above it keep the
+// times of claims ahead (RowClaims): 8,000 rows of 128 columns 66-71 us, 38 below it;
+// 20,000 rows 72-75 against 59.  At 16, GIN on 100,000 rows of 64 columns: 78 -> 84 us.
+inline bool small_plan(const cbm_plan* P, int team) {
+  return (P->n_items * team + 31) / 32 <= (int64_t)sm_count(P->device) * 24 * 8;
+}
+
 template <typename XT, typename YT, int VPL, int V, int FORM, int CLAIMS>
 int launch_fwd_claims(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
   // full-warp teams have their own instantiation (also where X's rows lie 2^32
@@ -69,13 +77,8 @@ int launch_fwd_claims(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
 
 template <typename XT, typename YT, int VPL, int V, int FORM>
 int launch_fwd_t(cbm_plan* P, const FwdArgs& a, cudaStream_t st) {
-  // Small plans: at most 8 groups for each warp of three blocks per SM (28,416 groups on
-  // B200).  With the line at one group or at three, the cases above it keep the
-  // times of claims ahead (RowClaims): 8,000 rows of 128 columns 66-71 us, 38 below it;
-  // 20,000 rows 72-75 against 59.  At 16, GIN on 100,000 rows of 64 columns: 78 -> 84 us.
   if constexpr (VPL <= 2 && FORM != FORM_COMP) {
-    const int64_t groups = ((int64_t)a.n_items * a.team + 31) / 32;
-    if (groups <= (int64_t)sm_count(P->device) * 24 * 8) {
+    if (small_plan(P, a.team)) {
       if (a.team >= 8) return launch_fwd_claims<XT, YT, VPL, V, FORM, CLAIMS_FEW>(P, a, st);
       if constexpr (VPL == 1) return launch_fwd_claims<XT, YT, VPL, V, FORM, CLAIMS_LONE>(P, a, st);
     }

@@ -504,18 +504,24 @@ int matmul_impl(cbm_plan* P, int32_t op, float gin_scale, const void* x, int32_t
     a.timeout_ns = P->timeout_ns;
     a.publish_epoch = 1;
     int s_team = 0, s_vpl = 0;
-    // AUTO takes the register kernel for rows of at most 32 vectors and on deep
-    // trees, the staged kernel for wider rows on shallow trees.  Measured on
-    // B200 (staged -> register, us): 800,000 nodes in 48 graphs, 64 BF16
-    // columns 944 -> 452; 200,000-node power-law graph, 32 / 64 / 128 FP32
-    // columns 397 / 380 / 313 -> 172 / 205 / 295; 1M nodes, 64 / 128 FP32
-    // columns 1332 / 1476 -> 936 / 1429; 400,000 nodes of mean degree 50, 128
-    // BF16 columns 1308 -> 1202.  256 FP32 columns: shallow 213 -> 297 and,
-    // with 1M nodes, 1943 -> 2702, deep (100,000 nodes, 84 % of the rows below
-    // level 0) 194 -> 167; 512 columns, deep 234 -> 180.
+    // AUTO takes the register kernel on shallow trees for rows of at most 32
+    // vectors (BF16 rows on larger plans 24: their 16 bytes are eight sums, and a full
+    // warp's rows have no registers left for them), on deep ones up to 128 (512
+    // FP32 columns: eight vectors per lane run at two to four warps per scheduler);
+    // the staged kernel for the others.  Measured on B200, staged -> register (us):
+    // shallow, 32 vectors and fewer: 800,000 nodes in 48 graphs, 64 BF16 columns 944
+    // -> 405; 200,000-node power-law graph, 32 / 64 / 128 FP32 columns 397 / 380 / 313 ->
+    // 172 / 205 / 280; 1M nodes, 64 / 128 FP32 columns 1332 / 1476 -> 936 / 1429; 400,000
+    // nodes of mean degree 50, 128 BF16 columns 1308 -> 992.  BF16, shallow, FP32 results:
+    // 192 / 208 / 256 columns on 60,000 nodes 143 / 146 / 141 -> 139 / 143 / 144, 200,000
+    // 364 / 375 / 355 -> 358 / 378 / 378; 208 / 256 on 1M 1696 / 1592 -> 1866 / 1873; 256 on a
+    // small plan, 20,000 nodes 87 -> 67.  FP32, 256 columns on 1M nodes 1943 -> 2702.
+    // Deep (GCN graph): 512 / 576 / 1,024 FP32 columns on 60,000 nodes 235 / 295 / 360 ->
+    // 182 / 384 / 450, on 170,000 639 / 789 / 1041 -> 556 / 1199 / 1399; 1,024 BF16 928 -> 700.
     // The GIN form runs on the register kernel (its self term and state rows
     // stay out of the staged kernel's registers).
-    const bool narrow = nvec <= 32 || P->deep;
+    const bool few = vpl <= 2 && small_plan(P, team);
+    const bool narrow = nvec <= (P->deep ? 128 : xdt == CBM_BF16 && !few ? 24 : 32);
     // Two passes (FP32 Y, no GIN term, no compensation): every row's delta sum
     // first, with no parent waits, then the parent terms in level order
     // (prop_kernel).  Opt-in: AUTO keeps the fused pass, which measured as

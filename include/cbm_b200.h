@@ -163,9 +163,9 @@ int cbm_plan_set_multipliers(cbm_plan* plan, const float* d_multipliers, void* s
  * in the staged kernel (0: its default; several streams share each warp).
  * Changing chunk_nnz or hot_rows re-lays out the plan (synchronous). */
 enum {
-  CBM_VARIANT_AUTO = 0,     /* staged for aligned rows of more than 32 16-byte vectors
-                               unless most rows hang below tree level 0, else register
-                               gather */
+  CBM_VARIANT_AUTO = 0,     /* register gather; staged for aligned rows of more than 32
+                               16-byte vectors (BF16 X, but on small plans: 24), 128 where
+                               most rows hang below tree level 0 */
   CBM_VARIANT_REGISTER = 1, /* X rows gathered into registers, U entries at a time */
   CBM_VARIANT_STAGED = 2,   /* X rows staged through shared memory by cp.async */
   CBM_VARIANT_TMA = 3       /* X rows gathered four at a time by TMA (tile::gather4) into
