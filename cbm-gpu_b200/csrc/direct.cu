@@ -394,11 +394,16 @@ __global__ void __launch_bounds__(kDirectThreads, 4) direct_spmm(const DirectArg
   constexpr int kTeams = kDirectThreads / TL;
   constexpr int kPerWarp = 32 / TL;  // rows of one row task
   // rows per run: one per team, up to four where every block then still gets
-  // several runs.  Runs are claimed in turn in the forms with a tree, whose
+  // several runs, fewer (whole warps' shares) where the rows would else leave
+  // blocks without one (2,215 rows, 8 columns: 65 us with a block's full run of 128
+  // rows, 38 with 16).  Runs are claimed in turn in the forms with a tree, whose
   // calls own the workspace (direct_mark zeroed the counter); the others may
   // share it with products on other streams and deal their runs out instead.
   const int64_t per_team = a.n_rows / ((int64_t)gridDim.x * kTeams * 4);
-  const int run = kTeams * (int)(TL < 4 || per_team < 1 ? 1 : per_team < 4 ? per_team : 4);
+  const int64_t shares = (a.n_rows + (int64_t)gridDim.x * kPerWarp - 1) / ((int64_t)gridDim.x * kPerWarp);
+  const int run = shares < kTeams / kPerWarp
+                      ? kPerWarp * (int)shares
+                      : kTeams * (int)(TL < 4 || per_team < 1 ? 1 : per_team < 4 ? per_team : 4);
   const int lane = threadIdx.x & 31;
   const int tl = lane % TL;
   float* ring = rings + (threadIdx.x >> 5) * kRingFloats;
