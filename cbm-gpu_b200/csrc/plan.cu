@@ -485,9 +485,17 @@ int cbm_plan_create(const int32_t* row_ptr, const int32_t* col_idx, const float*
     auto presummed = [&](int32_t v) { return pre && depth[v] > 0 && entries(v) >= kPreLen; };
     // entry groups a row's team steps through when its turn comes
     auto cost = [&](int32_t v) { return presummed(v) ? 1 : (entries(v) + 3) / 4; };
-    for (int32_t l = 0; l <= max_depth; ++l)
-      std::stable_sort(order.begin() + lvl_start[l], order.begin() + lvl_start[l + 1],
-                       [&](int32_t x, int32_t y) { return cost(x) > cost(y); });
+    std::vector<int32_t> level;
+    std::vector<int64_t> at;
+    for (int32_t l = 0; l <= max_depth; ++l) {
+      level.assign(order.begin() + lvl_start[l], order.begin() + lvl_start[l + 1]);
+      int32_t most = 0;
+      for (int32_t v : level) most = std::max(most, cost(v));
+      at.assign(most + 2, lvl_start[l]);
+      for (int32_t v : level) at[most - cost(v) + 1]++;
+      for (int32_t k = 0; k <= most; ++k) at[k + 1] += at[k] - lvl_start[l];
+      for (int32_t v : level) order[at[most - cost(v)]++] = v;
+    }
     for (int64_t i = 0; i < n_rows; ++i) P->pre_row[i] = presummed(order[i]);
   }
   std::vector<char> has_child(n_rows, 0);
