@@ -8,7 +8,7 @@
 // keep no state between calls, so neither do these: every call reads the
 // caller's arrays directly (no plan, no re-layout, no upload).  The only
 // memory they need beyond their operands is a caller-owned workspace of
-// 256 + 8 N bytes: a status word and a claim counter, and per node a
+// 256 + 8 N bytes: a status word and claim counters, and per node a
 // "has a parent" stamp and a "row is final" stamp.  Stamps are compared with a
 // per-call value from a process-wide counter, so the workspace is never
 // cleared between calls (it must be zero-filled once, before its first use).
@@ -16,11 +16,12 @@
 // Kernels (all on the caller's stream, none synchronises):
 //   direct_mark    every tree edge: stamp its child; check indices, that no
 //                  node has two parents and that the branch offsets are a
-//                  prefix sum ending at the edge count; zero the claim counter.
+//                  prefix sum ending at the edge count; zero the claim counters.
 //   direct_spmm    Y[i] = sum_k val_k X[col_k] over row i's entries in order
 //                  (one FMA per entry, the order of the oracle's restatement;
-//                  MKL's own summation order may differ in the last bits), a
-//                  team of lanes per row with 16-byte gathers of X rows;
+//                  MKL's own summation order may differ in the last bits):
+//                  long rows by column slices through cp.async rings, a team
+//                  of lanes for each other row, 16-byte gathers of X rows;
 //                  optionally + (1 + eps) X[i] fused into the store.
 //   direct_update  tree edges claimed in their listed order (parents precede
 //                  children in BFS order, so the earliest unfinished edge

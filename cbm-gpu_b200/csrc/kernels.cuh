@@ -509,71 +509,71 @@ __device__ __forceinline__ void gather_row(float (&acc)[VPL][V], const Lane<XT, 
       }
     }
   } else {
-  for (int b = 0; b < wlen; b += TL) {
-    const int in = b + TL + tl;
-    uint32_t en = 0;
-    float sn = 0.f;
-    if (in < len) {
-      en = __ldg(ent + in);
-      if (vals) sn = __ldg(vals + in);
-    }
-    const uint32_t c = e & kColMask;
-    const int cnt = len - b < TL ? len - b : TL;   // this team's entries in the batch (<= 0: none)
-    const int wc = wlen - b < TL ? wlen - b : TL;  // the warp's
-    typename R::type raw[U][VPL];
-    auto load = [&](int j, int u) {
-      const char* row = ln.row(__shfl_sync(0xffffffffu, c, j + u, TL));
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) raw[u][v] = R::load(reinterpret_cast<const XT*>(row + ln.off[v]));
-    };
-    auto add = [&](float su, int u) {
-#pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        float t[V];
-        R::widen(raw[u][v], t);
-#pragma unroll
-        for (int k = 0; k < V; ++k) acc[v][k] = fmaf(su, t[k], acc[v][k]);
+    for (int b = 0; b < wlen; b += TL) {
+      const int in = b + TL + tl;
+      uint32_t en = 0;
+      float sn = 0.f;
+      if (in < len) {
+        en = __ldg(ent + in);
+        if (vals) sn = __ldg(vals + in);
       }
-    };
-    auto after_loads = [&](int j) {
-      if (b + j == 0) {
-        between();
-        s = __fmul_rn(s, dv);
-      }
-    };
-    int j = 0;
-    if (TLC == 32) {
-      // whole groups without predicates
-#pragma unroll 1
-      for (; j + U <= cnt; j += U) {
-#pragma unroll
-        for (int u = 0; u < U; ++u) load(j, u);
-        after_loads(j);
-#pragma unroll
-        for (int u = 0; u < U; ++u) add(__shfl_sync(0xffffffffu, s, j + u, TL), u);
-      }
-    }
-#pragma unroll 1
-    for (; j < wc; j += U) {
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
+      const uint32_t c = e & kColMask;
+      const int cnt = len - b < TL ? len - b : TL;   // this team's entries in the batch (<= 0: none)
+      const int wc = wlen - b < TL ? wlen - b : TL;  // the warp's
+      typename R::type raw[U][VPL];
+      auto load = [&](int j, int u) {
         const char* row = ln.row(__shfl_sync(0xffffffffu, c, j + u, TL));
-        if (j + u < cnt) {
 #pragma unroll
-          for (int v = 0; v < VPL; ++v) raw[u][v] = R::load(reinterpret_cast<const XT*>(row + ln.off[v]));
+        for (int v = 0; v < VPL; ++v) raw[u][v] = R::load(reinterpret_cast<const XT*>(row + ln.off[v]));
+      };
+      auto add = [&](float su, int u) {
+#pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          float t[V];
+          R::widen(raw[u][v], t);
+#pragma unroll
+          for (int k = 0; k < V; ++k) acc[v][k] = fmaf(su, t[k], acc[v][k]);
+        }
+      };
+      auto after_loads = [&](int j) {
+        if (b + j == 0) {
+          between();
+          s = __fmul_rn(s, dv);
+        }
+      };
+      int j = 0;
+      if (TLC == 32) {
+        // whole groups without predicates
+#pragma unroll 1
+        for (; j + U <= cnt; j += U) {
+#pragma unroll
+          for (int u = 0; u < U; ++u) load(j, u);
+          after_loads(j);
+#pragma unroll
+          for (int u = 0; u < U; ++u) add(__shfl_sync(0xffffffffu, s, j + u, TL), u);
         }
       }
-      after_loads(j);
+#pragma unroll 1
+      for (; j < wc; j += U) {
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float su = __shfl_sync(0xffffffffu, s, j + u, TL);
-        if (j + u < cnt) add(su, u);
+        for (int u = 0; u < U; ++u) {
+          const char* row = ln.row(__shfl_sync(0xffffffffu, c, j + u, TL));
+          if (j + u < cnt) {
+#pragma unroll
+            for (int v = 0; v < VPL; ++v) raw[u][v] = R::load(reinterpret_cast<const XT*>(row + ln.off[v]));
+          }
+        }
+        after_loads(j);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const float su = __shfl_sync(0xffffffffu, s, j + u, TL);
+          if (j + u < cnt) add(su, u);
+        }
       }
+      e = en;
+      if (!vals) sn = in < len ? reg_scale(en, vals, in, scale_mode, mult) : 0.f;
+      s = __fmul_rn(sn, dv);
     }
-    e = en;
-    if (!vals) sn = in < len ? reg_scale(en, vals, in, scale_mode, mult) : 0.f;
-    s = __fmul_rn(sn, dv);
-  }
   }
 }
 
@@ -668,7 +668,8 @@ static_assert(chunk_stop(INT_MAX, kPreMark) == INT_MAX && chunk_stop(5, 12) == 5
 enum RowForm : int { FORM_PLAIN = 0, FORM_GIN = 1, FORM_COMP = 2 };
 
 template <typename XT, typename YT, int VPL, int V, int FORM, int TLC, int CLAIMS>
-__global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, TLC, CLAIMS>())) fwd_kernel(const FwdArgs a) {
+__global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, TLC, CLAIMS>()))
+    fwd_kernel(const FwdArgs a) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr bool COMP = FORM == FORM_COMP;
   constexpr bool kPlain = FORM == FORM_PLAIN;
@@ -2179,45 +2180,45 @@ __device__ __forceinline__ void gather_dual_row(float (&acc)[S][VPL][V], const L
       }
     }
   } else {
-  for (int b = 0; b < wlen; b += TL) {
-    const int at = b + TL + tl;
-    const uint32_t en = at < len ? __ldg(ent + at) : 0u;
-    const int cnt = len - b < TL ? len - b : TL;
-    const int wc = wlen - b < TL ? wlen - b : TL;
+    for (int b = 0; b < wlen; b += TL) {
+      const int at = b + TL + tl;
+      const uint32_t en = at < len ? __ldg(ent + at) : 0u;
+      const int cnt = len - b < TL ? len - b : TL;
+      const int wc = wlen - b < TL ? wlen - b : TL;
 #pragma unroll 1
-    for (int j = 0; j < wc; j += U) {
-      typename D::type raw[U][VPL];
-      uint32_t eu[U];
+      for (int j = 0; j < wc; j += U) {
+        typename D::type raw[U][VPL];
+        uint32_t eu[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        eu[u] = __shfl_sync(0xffffffffu, e, j + u, TL);
-        const uint32_t r = eu[u] & kIndexMask;
-        const bool in = (eu[u] & kInternalBit) != 0;
-        if (j + u < cnt) {
-          const char* g = lg.row(r);
-          const char* h = lh.row(r);
+        for (int u = 0; u < U; ++u) {
+          eu[u] = __shfl_sync(0xffffffffu, e, j + u, TL);
+          const uint32_t r = eu[u] & kIndexMask;
+          const bool in = (eu[u] & kInternalBit) != 0;
+          if (j + u < cnt) {
+            const char* g = lg.row(r);
+            const char* h = lh.row(r);
 #pragma unroll
-          for (int v = 0; v < VPL; ++v) raw[u][v] = D::load(g + lg.off[v], h + lh.off[v], in);
+            for (int v = 0; v < VPL; ++v) raw[u][v] = D::load(g + lg.off[v], h + lh.off[v], in);
+          }
         }
-      }
-      if (b + j == 0) between();
+        if (b + j == 0) between();
 #pragma unroll
-      for (int u = 0; u < U; ++u) {
-        const float su = __shfl_sync(0xffffffffu, s, j + u, TL);
-        if (j + u < cnt) {
+        for (int u = 0; u < U; ++u) {
+          const float su = __shfl_sync(0xffffffffu, s, j + u, TL);
+          if (j + u < cnt) {
 #pragma unroll
-          for (int v = 0; v < VPL; ++v) {
-            float t[V];
-            D::widen(raw[u][v], (eu[u] & kInternalBit) != 0, t);
+            for (int v = 0; v < VPL; ++v) {
+              float t[V];
+              D::widen(raw[u][v], (eu[u] & kInternalBit) != 0, t);
 #pragma unroll
-            for (int k = 0; k < V; ++k) acc[u % S][v][k] = fmaf(su, t[k], acc[u % S][v][k]);
+              for (int k = 0; k < V; ++k) acc[u % S][v][k] = fmaf(su, t[k], acc[u % S][v][k]);
+            }
           }
         }
       }
+      e = en;
+      s = at < len ? dual_scale(en, scale_g, mult) : 0.f;
     }
-    e = en;
-    s = at < len ? dual_scale(en, scale_g, mult) : 0.f;
-  }
   }
 }
 

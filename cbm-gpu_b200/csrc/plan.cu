@@ -6,7 +6,8 @@
 // (cbm/cbm.cu:181,203).  A plan instead owns one device copy of the structure
 // laid out for the fused kernel:
 //
-//   items    rows sorted by tree depth (stable by node id): the work queue order
+//   items    rows sorted by tree depth, on deep trees by length inside a level,
+//            else by node id: the work queue order
 //   ent      column | sign << 31 of every delta entry, rows in item order
 //   ptr      int64 offsets of each item's entries
 //   par      parent node per item (-1 for children of the virtual root)
