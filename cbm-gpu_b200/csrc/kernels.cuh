@@ -851,15 +851,14 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
 
     // ---- the row's end: chunk partials, parent, store, ready flag
     const bool near_any = TLC != 32 && __any_sync(kAll, have && (m0.x & kNearBit) != 0);
-    bool todo = have, more = false;
-    int turn = 0;
+    const int turns = AHEAD && !near_any ? 1 : AHEAD ? (int)teams : INT_MAX;
+    bool todo = have;
     unsigned long long t0 = 0;
-    do {
+    for (int turn = 0; turn < turns; ++turn) {
       bool go = todo;
       if constexpr (AHEAD) {
         // a group that may hold an item and its parent: team by team, in queue order
-        go = have && (!near_any || team == turn);
-        more = near_any && ++turn < (int)teams;
+        go = have && (turns == 1 || team == turn);
       } else if (near_any) {
         // here those whose parent is ready
         if (go && p >= 0) go = ld_acquire(a.node_flag + p) == epoch;
@@ -1004,8 +1003,8 @@ __global__ void __launch_bounds__(kThreads, (fwd_min_blocks<XT, YT, VPL, FORM, T
         }
       }
       __syncwarp();
-      if constexpr (!AHEAD) more = near_any && __any_sync(kAll, todo);
-    } while (more);
+      if (!AHEAD && !(near_any && __any_sync(kAll, todo))) break;
+    }
     // ---- on to the next row: its entries are here, the record behind it loads
     if constexpr (!AHEAD) {
       begin();
