@@ -647,11 +647,11 @@ __device__ __forceinline__ void finish_block(QueueState* qs, unsigned epoch, boo
 // the presummed rows and kPreMark.
 //
 // Measured on B200 against one row per claim and warp with every load in turn
-// (bit-identical): 170,000-node GCN graph, 128 FP32 columns 262 -> 163 us, 128
-// BF16 210 -> 146, 40 BF16 174 -> 116; 100,000 nodes, 47 FP32 columns (no
-// 16-byte vectors) 273 -> 104, GIN with 64 columns 122 -> 79.  What is left is
+// (bit-identical): 170,000-node GCN graph, 128 FP32 columns 259 -> 160 us, 128
+// BF16 208 -> 145, 40 BF16 174 -> 102-115; 100,000 nodes, 47 FP32 columns (no
+// 16-byte vectors) 272 -> 103, GIN with 64 columns 120 -> 77.  What is left is
 // instruction issue and the exposed round trip per row, not bandwidth: no
-// gather at all leaves 66 us of the first (profiled by leaving parts out).
+// gather at all leaves 66 us of the first (timed by leaving parts out).
 constexpr int kNearBit = 0x40000000;
 constexpr int kNodeMask = 0x3fffffff;
 // null records past the last item: a group there starts at item n at most
